@@ -229,7 +229,7 @@ ohm_status ohm_solve_real_device(ohm_ctx *ctx, const ohm_csr *a, const ohm_buf *
  * calls neither.  The caller passes device pointers for the CSR, b and the
  * output x, and the stream to run on (NULL = the default stream), on the
  * current device.  All other working memory is one fixed file-scope device
- * array of about 6.2 MB, held by every GPU that loads the library until the
+ * array of about 7.3 MB, held by every GPU that loads the library until the
  * process exits; systems above 32768 rows or 262144 nonzeros are rejected
  * with OHM_ERR_INVALID_ARG.  The first call on a device looks up that
  * device's address of the array: make it before any stream capture.  Every

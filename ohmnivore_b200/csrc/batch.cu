@@ -178,8 +178,11 @@ extern "C" ohm_status ohm_batch_create(ohm_ctx *c, int64_t n_inst, const int64_t
     if (any_pair) { PUT(u8, flag.data(), rows); a.rowflag = u8; }
     ZERO(f64, 4 * rows); a.rec0 = f64;
     ZERO(f64, 4 * rows); a.rec1 = f64;
-    void **vs[] = {&a.rhat, &a.s, &a.t, &a.phat, &a.shat, &a.d, &a.pc_part};
+    void **vs[] = {&a.rhat, &a.s, &a.t, &a.phat, &a.shat, &a.d, &a.pc_part, &a.cself, &a.rself};
     for (void **slot : vs) { ZERO(f64, rows); *slot = f64; }
+    { uint16_t *lc = nullptr; PUT(lc, (const uint16_t *)nullptr, nnz + nnz / 4); a.slice_col = lc; }
+    { double *lv = nullptr; PUT(lv, (const double *)nullptr, nnz + nnz / 4); a.slice_val = lv; }
+    { uint8_t *ex = nullptr; PUT(ex, (const uint8_t *)nullptr, rows); a.slice_export = ex; }
     DiodeDesc *dd = nullptr; PUT(dd, (const DiodeDesc *)diodes, nd); a.diodes = dd;
     BjtDesc *qd = nullptr; PUT(qd, (const BjtDesc *)bjts, nq); a.bjts = qd;
     MosfetDesc *md = nullptr; PUT(md, (const MosfetDesc *)mosfets, nm); a.mosfets = md;

@@ -65,6 +65,11 @@ __host__ __device__ inline void instance_args(const BatchArgs &B, int i, const I
     a.phat = (double *)B.base.phat + ro;
     a.shat = (double *)B.base.shat + ro;
     a.d = (double *)B.base.d + ro;
+    a.cself = (double *)B.base.cself + ro;
+    a.rself = (double *)B.base.rself + ro;
+    a.slice_col = offset(B.base.slice_col, no + no / 4);
+    a.slice_val = offset(B.base.slice_val, no + no / 4);
+    a.slice_export = offset(B.base.slice_export, ro);
     a.nd = (int)(o.dq1 - dq);
     a.nq = (int)(o.qq1 - qq);
     a.nm = (int)(o.mq1 - mq);
@@ -90,9 +95,10 @@ __host__ __device__ inline void instance_args(const BatchArgs &B, int i, const I
 }
 
 template <int LPR, int BLOCK, int MINB>
-__global__ void __launch_bounds__(BLOCK, MINB) batch_solver(BatchArgs B) {
+__global__ void __launch_bounds__(BLOCK, MINB) batch_solver(const __grid_constant__ BatchArgs B) {
     __shared__ double smem[32 * 4];
     __shared__ int s_q;
+    reduce_buffers_init();
     for (;;) {
         if (threadIdx.x == 0) s_q = (int)atomicAdd(B.queue, 1u);
         __syncthreads();
@@ -115,6 +121,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) batch_solver(BatchArgs B) {
         g.gtid = threadIdx.x;
         g.gstride = blockDim.x;
         g.smem = smem;
+        g.map.state = kSliceNone;
         solve_body<LPR>(a, g, &B.infos[i]);
         __syncthreads();
     }

@@ -12,6 +12,21 @@
 
 using ohm::DeviceInfo;
 
+// The persistent solver per lanes per row, instantiated in solver_k*.cu.
+using KernelFn = void (*)(ohm::KernelArgs);
+template <int LPR>
+KernelFn persistent_kernel_for();
+template <>
+KernelFn persistent_kernel_for<1>();
+template <>
+KernelFn persistent_kernel_for<4>();
+template <>
+KernelFn persistent_kernel_for<8>();
+template <>
+KernelFn persistent_kernel_for<16>();
+template <>
+KernelFn persistent_kernel_for<32>();
+
 // Records the message for ohm_last_error() and returns `st`.
 ohm_status ohm_fail(ohm_status st, const char *fmt, ...);
 
@@ -52,9 +67,34 @@ struct LaunchTarget {
 ohm_status ohm_launch_persistent(const LaunchTarget &t, ohm::KernelArgs &a, int64_t nnz, int *launches);
 ohm_status ohm_finish_persistent(const LaunchTarget &t, ohm_solve_info *info, int launches);
 ohm_status ohm_check_krylov(const ohm_krylov_params *p);
-// Dynamic shared memory that lets a grid-team kernel `fn` of `grid` blocks
-// keep its Krylov slices in shared memory (sets the kernel's limit), or 0.
-int ohm_krylov_smem_bytes(const void *fn, int64_t n, int64_t nnz_short, int grid);
+// Grid, dynamic shared memory (a.smem_bytes) and synchronisation (a.cluster)
+// of a grid-team kernel `fn` over a.n rows; `slices`: keep Krylov slices in
+// shared memory.
+constexpr int kMaxTeamCluster = 16, kTeamRows = 1024;
+ohm_status ohm_team_shape(const void *fn, int num_sms, int max_grid, bool slices, int64_t nnz, ohm::KernelArgs &a,
+                          int &grid);
+// Launch configuration of that shape: one cluster, or a cooperative grid.
+struct TeamLaunch {
+    cudaLaunchConfig_t config = {};
+    cudaLaunchAttribute attr[1] = {};
+    TeamLaunch(int grid, const ohm::KernelArgs &a, cudaStream_t stream) {
+        config.gridDim = dim3(grid);
+        config.blockDim = dim3(ohm::kSolverBlock);
+        config.dynamicSmemBytes = (size_t)a.smem_bytes;
+        config.stream = stream;
+        if (a.cluster) {
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = grid;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        } else {
+            attr[0].id = cudaLaunchAttributeCooperative;
+            attr[0].val.cooperative = 1;
+        }
+        config.attrs = attr;
+        config.numAttrs = 1;
+    }
+    TeamLaunch(const TeamLaunch &) = delete;
+};
 // Kernel arguments of a Newton solve on a plan (validated params), its
 // context, and the launch of a plan-sized persistent kernel (api.cu).
 ohm_status ohm_plan_kernel_args(ohm_plan *p, const ohm_newton_params *np, double *x_dev, ohm::KernelArgs &a,

@@ -8,7 +8,7 @@
 // passes device-resident inputs and the output vector; every other byte the
 // solve needs comes from one file-scope __device__ array of fixed size.
 //
-// Limits: at most kMaxRows rows and kMaxNnz nonzeros (about 6.2 MB of device
+// Limits: at most kMaxRows rows and kMaxNnz nonzeros (about 7.3 MB of device
 // memory, held by every GPU that loads this library until the process exits).
 // Set-up: the first call on a device looks up that device's address of the
 // array (cudaGetSymbolAddress, with the device current); make that first call
@@ -37,8 +37,8 @@ constexpr int kMaxDevices = 64;
 constexpr size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // Scratch layout (byte offsets), each region 256-byte aligned.
-constexpr size_t kOffVec = 0;                                               // 15 x rows x 8
-constexpr size_t kOffR64 = kOffVec + align256(15 * kMaxRows * 8);
+constexpr size_t kOffVec = 0;                                               // 17 x rows x 8
+constexpr size_t kOffR64 = kOffVec + align256(17 * kMaxRows * 8);
 constexpr size_t kOffDx = kOffR64 + align256(kMaxRows * 8);
 constexpr size_t kOffPartials = kOffDx + align256(kMaxRows * 8);            // 8 x grid doubles
 constexpr size_t kOffPartner = kOffPartials + align256(8 * kMaxGrid * 8);
@@ -48,7 +48,9 @@ constexpr size_t kOffCand = kOffOff + align256(kMaxRows * 4);
 constexpr size_t kOffChoice = kOffCand + align256(kMaxRows * 4);
 constexpr size_t kOffFlag = kOffChoice + align256(kMaxRows * 4);
 constexpr size_t kOffVals32 = kOffFlag + align256(kMaxRows);
-constexpr size_t kOffSync = kOffVals32 + align256(kMaxNnz * 4);            // 4 words + check flag
+constexpr size_t kOffSliceCol = kOffVals32 + align256(kMaxNnz * 4);
+constexpr size_t kOffExport = kOffSliceCol + align256(kMaxNnz * 2);
+constexpr size_t kOffSync = kOffExport + align256(kMaxRows);                 // 4 words + check flag
 constexpr size_t kOffInfo = kOffSync + 256;
 constexpr size_t kScratchBytes = kOffInfo + align256(sizeof(DeviceInfo));
 
@@ -244,8 +246,10 @@ extern "C" ohm_status ohm_solve_real_noalloc(void *stream, int64_t n, int64_t nn
     double *vec = (double *)(base + kOffVec);
     a.rec0 = (void *)vec;
     a.rec1 = (void *)(vec + 4 * (size_t)n);
-    void **slots[] = {&a.rhat, &a.s, &a.t, &a.phat, &a.shat, &a.d, &a.pc_part};
-    for (int k = 0; k < 7; ++k) *slots[k] = (void *)(vec + (8 + (size_t)k) * n);
+    a.slice_col = (uint16_t *)(base + kOffSliceCol);
+    a.slice_export = (uint8_t *)(base + kOffExport);
+    void **slots[] = {&a.rhat, &a.s, &a.t, &a.phat, &a.shat, &a.d, &a.pc_part, &a.cself, &a.rself};
+    for (int k = 0; k < 9; ++k) *slots[k] = (void *)(vec + (8 + (size_t)k) * n);
     a.r64 = (double *)(base + kOffR64);
     a.dx = (double *)(base + kOffDx);
     a.partials = (double *)(base + kOffPartials);

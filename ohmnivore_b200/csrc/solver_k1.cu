@@ -1,0 +1,5 @@
+// Persistent solver, 1 lane(s) per row.
+#include "internal.cuh"
+
+template <>
+KernelFn persistent_kernel_for<1>() { return ohm::persistent_solver<1>; }

@@ -1,0 +1,5 @@
+// Persistent solver, 16 lane(s) per row.
+#include "internal.cuh"
+
+template <>
+KernelFn persistent_kernel_for<16>() { return ohm::persistent_solver<16>; }

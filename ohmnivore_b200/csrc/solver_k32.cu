@@ -1,0 +1,5 @@
+// Persistent solver, 32 lane(s) per row.
+#include "internal.cuh"
+
+template <>
+KernelFn persistent_kernel_for<32>() { return ohm::persistent_solver<32>; }

@@ -56,9 +56,13 @@ enum SolveStatus : int {
 
 enum PrecondKind : int { kPcAuto = 0, kPcJacobi = 1, kPcIsai = 2, kPcNone = 3 };
 
-// Threads per block of the persistent solver (one block per SM).
+// Threads per block of the persistent solver (one block per SM).  512 threads
+// have 128 registers each and half the per-warp overhead of a phase (barriers,
+// reductions, address arithmetic) of 1024 threads with 64: DC of the 500 x 500
+// diode mesh 382 -> 234 ms, of a 100 x 100 one 31.7 -> 24.7 ms (256 threads:
+// 276 and 26.5 ms).
 #ifndef OHM_SOLVER_BLOCK
-#define OHM_SOLVER_BLOCK 1024
+#define OHM_SOLVER_BLOCK 512
 #endif
 constexpr int kSolverBlock = OHM_SOLVER_BLOCK;
 
@@ -181,11 +185,19 @@ struct KernelArgs {
     double *partials;           // >= 8 * gridDim.x doubles (two alternating regions)
     GridSync gs;
     DeviceInfo *info;
-    // dynamic shared memory of the launch (grid-team kernels): when > 0 the
-    // Krylov solve keeps each block's slice there if it fits (krylov()).
-    // nnz_long: nonzeros of the long rows (host side, sizes that slice).
+    // dynamic shared memory of the launch: when > 0 the Krylov solve keeps each
+    // block's slice there as far as it fits (krylov_slice()).  nnz_long:
+    // nonzeros of the long rows (host side, sizes that slice).  cluster: the
+    // grid is one thread-block cluster.  slice_col and slice_val (5
+    // entries per 4 nonzeros), slice_export (u8 per row), cself and rself (8
+    // bytes per row) are that solve's workspace.
     int smem_bytes;
     int64_t nnz_long;
+    int cluster;
+    uint16_t *slice_col;
+    double *slice_val;
+    uint8_t *slice_export;
+    void *cself, *rself;
 };
 
 // Columns of the per-outer-iteration trace: FP32 Krylov iterations, FP64
@@ -193,42 +205,89 @@ struct KernelArgs {
 // used, max|x - x_old| after limiting, restarts.
 constexpr int kTraceCols = 6;
 
+// What a block knows about its slice of the system (krylov_slice()), built at
+// the first Krylov solve of a launch: H halo rows, matrix slices of 32 W entries.
+enum SliceState : int {
+    kSliceNone = 0,     // not built yet
+    kSliceChip = 1,     // everything in shared memory
+    kSliceStream = 2,   // gather vector in shared memory, matrix slices in global memory
+    kSliceCsr = 3,      // gather vector in shared memory, the CSR arrays in global memory
+    kSliceNo = 4,       // does not fit: global-memory solve
+};
+struct SliceMap {
+    int state, H, W, pairs;   // W: padded nonzeros / 32
+};
+
 // A team is the set of threads that solves one system: the whole grid (one
 // large circuit, GridTeam) or one block (one circuit of a batch, BlockTeam).
 // Both expose the rows this block owns [r0, r1), a thread index / stride over
 // the team for device- and slot-parallel loops, sync() and deterministic
 // all-reductions whose results are bit-identical in every thread.
+// A grid of one block synchronises within the block; a grid of up to 16
+// blocks is launched as one cluster and meets at cluster barriers with its
+// dot products exchanged through distributed shared memory; larger grids
+// meet at the counter barrier.  The sums have the same order in all three.
 struct GridTeam {
     int G, bid, r0, r1, gtid, gstride;
     double *smem;
     double *partials;
-    int red;
-    unsigned long long epoch;
+    bool cluster;
     GridSync gs;
+    SliceMap map;
 
-    __device__ __forceinline__ bool sync() { return grid_barrier(gs, epoch); }
-    __device__ __forceinline__ bool leader() const { return bid == 0 && threadIdx.x == 0; }
-    // Consecutive grid reductions alternate between two partial regions: a
-    // block may publish reduction j+1 while a slower block still reads
-    // reduction j, but never reduction j+2 (a barrier separates them).
-    __device__ __forceinline__ double *part() {
-        double *p = partials + (size_t)(red & 1) * 4 * G;
-        ++red;
-        return p;
+    __device__ __forceinline__ void init(const KernelArgs &a) {
+        G = gridDim.x;
+        bid = blockIdx.x;
+        r0 = (int)(((long long)a.n * bid) / G);
+        r1 = (int)(((long long)a.n * (bid + 1)) / G);
+        gtid = bid * blockDim.x + threadIdx.x;
+        gstride = G * blockDim.x;
+        smem = reduce_buffers().warp;
+        partials = a.partials;
+        cluster = a.cluster != 0;
+        gs = a.gs;
+        map.state = kSliceNone;
+        reduce_buffers_init();
+        if (cluster) cluster_barrier();     // peers' shared memory exists from here on
+    }
+    __device__ __forceinline__ bool sync() {
+        if (gridDim.x == 1) { __syncthreads(); return true; }
+        if (cluster) { cluster_barrier(); return true; }
+        return grid_barrier(gs);
+    }
+    __device__ __forceinline__ bool leader() const { return blockIdx.x == 0 && threadIdx.x == 0; }
+    template <int NV, bool MAX = false, typename Fin>
+    __device__ __forceinline__ bool reduce_then(const double (&v)[NV], Fin fin) {
+        return team_reduce_then<NV, MAX>((int)gridDim.x, cluster, partials, gs, v, fin);
+    }
+    template <int NV, bool MAX>
+    __device__ __forceinline__ bool reduce(double (&v)[NV]) {
+        double *res = reduce_buffers().res;
+        const bool ok = reduce_then<NV, MAX>(v, [&](const double (&t)[NV], bool writer) {
+            if (writer) {
+#pragma unroll
+                for (int k = 0; k < NV; ++k) res[k] = t[k];
+            }
+        });
+#pragma unroll
+        for (int k = 0; k < NV; ++k) v[k] = res[k];
+        return ok;
     }
     template <int NV>
-    __device__ __forceinline__ bool allreduce(double (&v)[NV]) {
-        return grid_allreduce<NV, false>(v, part(), gs, epoch, smem);
-    }
+    __device__ __forceinline__ bool allreduce(double (&v)[NV]) { return reduce<NV, false>(v); }
     template <int NV>
-    __device__ __forceinline__ bool allmax(double (&v)[NV]) {
-        return grid_allreduce<NV, true>(v, part(), gs, epoch, smem);
-    }
+    __device__ __forceinline__ bool allmax(double (&v)[NV]) { return reduce<NV, true>(v); }
 };
 
 struct BlockTeam {
     int r0, r1, gtid, gstride;
     double *smem;
+    SliceMap map;
+
+    template <int NV, bool MAX = false, typename Fin>
+    __device__ __forceinline__ bool reduce_then(const double (&v)[NV], Fin fin) {
+        return team_reduce_then<NV, MAX>(1, false, nullptr, GridSync{nullptr, nullptr}, v, fin);
+    }
 
     __device__ __forceinline__ bool sync() { __syncthreads(); return true; }
     __device__ __forceinline__ bool leader() const { return threadIdx.x == 0; }
@@ -251,9 +310,9 @@ __device__ __forceinline__ T cvt(double x) { return (T)x; }
 // block's local CSR slice has rp_off = its first row).
 constexpr int kRowsInFlight = 4;
 
-template <int LPR, typename Acc, typename TA, typename X, typename F, int U = kRowsInFlight, bool PIPE = false>
-__device__ __forceinline__ void spmv_rows(const uint32_t *__restrict__ rp,
-                                          const uint32_t *__restrict__ col,
+template <int LPR, typename Acc, typename TA, typename X, typename F, int U = kRowsInFlight, bool PIPE = false,
+          typename TR, typename TC>
+__device__ __forceinline__ void spmv_rows(const TR *__restrict__ rp, const TC *__restrict__ col,
                                           const TA *__restrict__ val, const uint8_t *rowflag,
                                           int r0, int r1, X x, F f, const uint8_t *skip = nullptr,
                                           int rp_off = 0) {
@@ -681,291 +740,644 @@ __device__ __forceinline__ int krylov(const KernelArgs &a, Team &g, double tol_f
 
 namespace ohm {
 
-// The slice of krylov_smem() does not fit in the launch's shared memory.
-constexpr int kKrylovNoSmem = -2;
+// krylov() with each block's slice of the system in shared memory.
+//
+// What bounds it: the working set sits on the chip, so an iteration is a
+// chain of latencies (three team reductions, and in each SpMV phase the round
+// trip to the neighbours' rows) and of issued instructions.  So:
+//   * each phase first forms the vector that the product gathers (M^-1 p or
+//     M^-1 s) once per row into shared memory, z: the block's own rows from
+//     its own state, the rows of other blocks that its nonzeros touch (the
+//     halo: about 1,000 rows for the 8,400 nonzeros of a 1,690-row slice of a
+//     500 x 500 mesh) from the records that their owners publish, every
+//     remote record fetched once and all of them at the same time;
+//   * the matrix is stored in slices of 32 rows padded to their longest row,
+//     entry k of the 32 rows side by side (16-bit local columns; padding has
+//     value 0 and the column of a zero): a warp's loads are consecutive, the
+//     product costs three shared-memory loads and an FMA per nonzero;
+//   * own-row state is one array per field (no bank conflicts), and only rows
+//     in someone's halo are published (slice_export);
+//   * the scalars of the recurrence live in shared memory and are updated by
+//     one lane inside the reductions (KrylovScalars): every thread repeating
+//     the divisions and square roots cost 300 of 1,350 instructions per warp
+//     and iteration, and the registers that held them were spilled.
+// Measured together with the cluster teams and the cheaper reductions (B200,
+// 512 threads a block), before -> after: DC of the 500 x 500 diode mesh (one
+// block per SM, 1,690 rows each) 340 -> 238 ms, 23.5 -> 16 us per BiCGSTAB
+// iteration; 100 x 100 mesh (a cluster of 10) 47 -> 27 ms; 600 x 600 mesh
+// (stream layout) 760 -> 473 ms; 200 steps of a 401-row transient (one block)
+// 116 -> 44 ms.
+// The values and their order are krylov()'s, so the results are bit-identical
+// (fma is written out where two phases share code: a product merged from two
+// branches is not contracted).
+//
+// Layouts, chosen per block when the slice map is built:
+//   chip   everything in shared memory;
+//   stream (larger slices) z and the vectors, in the order of their traffic,
+//          while they fit; the 32-row slices of the matrix in global memory;
+//   csr    (several lanes per row) vectors as in `stream`, the matrix read
+//          from its CSR arrays through local column indices;
+//   none   z does not fit, or the halo overflows its table: krylov().
+// A block chooses for itself: blocks exchange data only through the published
+// records and the reductions (one without a slice marks every column of its
+// rows for export).
+constexpr uint32_t kHaloPaired = 0x80000000u;    // halo entry: the row is half of a 2x2 pair
+constexpr uint8_t kRowPaired = 1, kRowExport = 2, kRowLong = 4;
 
-// krylov() with each block's slice in shared memory: the CSR rows it owns
-// (local row pointers, columns, values in the Krylov precision; long rows
-// stay with the team), its rows' records, r_hat, t, d, the Newton weights
-// and a pair flag.  Every phase then reads global memory only for the
-// neighbours' records that the SpMV gathers, and the own-row updates touch
-// shared memory (addressed with 32-bit offsets) plus the published record
-// fields.  The arithmetic and its order are krylov()'s, so the results are
-// the same.  The slice is laid out per solve (the values change with every
-// Newton iteration); a block whose slice does not fit returns kKrylovNoSmem
-// before touching anything, and the caller runs krylov() (a per-block
-// choice: blocks exchange data only through the global records and the
-// reductions).  U rows per group are in flight in each SpMV tile.
-template <typename T, int LPR, int U>
-__device__ __forceinline__ int krylov_smem(const KernelArgs &a, GridTeam &g, double tol_floor, double inner_rtol,
-                                           int max_it, bool accept_partial, KrylovOut &out) {
-    using Acc = T;
+__device__ __forceinline__ uint32_t up16(uint32_t x) { return (x + 15u) & ~15u; }
+
+// Byte offsets in dynamic shared memory: slice starts at 0, halo list, row
+// flags, columns of the matrix slices (32 W entries; none when they are in
+// global memory), z (R + H rows and a zero), eight own-row vectors of eight
+// bytes a row in either Krylov precision, values of the matrix slices.
+struct SliceOffsets {
+    uint32_t halo, flag, col, z, vec, vec_bytes, val, end;
+};
+__device__ __forceinline__ SliceOffsets slice_offsets(uint32_t R, uint32_t H, uint32_t W) {
+    SliceOffsets o;
+    o.halo = up16(4u * ((R + 31u) / 32u + 1u));
+    o.flag = o.halo + up16(4u * H);
+    o.col = o.flag + up16(R);
+    o.z = o.col + 64u * W;
+    o.vec = o.z + up16(8u * (R + H + 1u));
+    o.vec_bytes = up16(8u * R);
+    o.val = o.vec + 8u * o.vec_bytes;
+    o.end = o.val + 256u * W;
+    return o;
+}
+
+template <class Team>
+__device__ __forceinline__ bool team_of_one(const Team &g) {
+    if constexpr (std::is_same<Team, GridTeam>::value) return g.G == 1;
+    else return true;
+}
+
+// Room for the padded matrix slices of nonzeros [k0, k1) in global memory
+// (slice_val / slice_col hold 5 entries for every 4 nonzeros).
+__device__ __forceinline__ uint32_t slice_start(uint32_t k) { return k + k / 4u; }
+
+// Builds the block's slice map (once per launch; once per circuit in a
+// batch): halo rows numbered through a hash table at the top of the dynamic
+// shared memory, row flags, matrix slices' columns.  Returns false when a
+// team sync gave up.
+template <int LPR, class Team>
+__device__ __forceinline__ bool slice_map(const KernelArgs &a, Team &g) {
+    __shared__ int s_count, s_fail;
     const int r0 = g.r0, r1 = g.r1, R = r1 - r0;
-    if (a.smem_bytes == 0 || R <= 0) return kKrylovNoSmem;
-    const T *A;
-    if constexpr (sizeof(T) == 4) A = (const T *)a.vals32; else A = (const T *)a.vals64;
-    const bool wt = a.newton != 0;
-    // ---- layout: local row pointers by a block scan over contiguous chunks ----
-    const int chunk = (R + (int)blockDim.x - 1) / (int)blockDim.x;
-    const int c0 = min(R, (int)threadIdx.x * chunk), c1 = min(R, c0 + chunk);
-    uint32_t mine = 0;
-    for (int li = c0; li < c1; ++li) {
-        const int i = r0 + li;
-        if (!(a.longflag != nullptr && a.longflag[i] != 0)) mine += a.row_ptr[i + 1] - a.row_ptr[i];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const bool lone = team_of_one(g), pairs = a.precond == kPcAuto;
+    SliceMap m{kSliceNo, 0, 0, 0};
+    g.map = m;
+    if (a.smem_bytes == 0) return true;      // uniform over the team
+    const uint32_t room = (uint32_t)a.smem_bytes & ~15u;
+    auto row_len = [&](int i) -> uint32_t {
+        if (a.longflag != nullptr && a.longflag[i] != 0) return 0u;
+        return a.row_ptr[i + 1] - a.row_ptr[i];
+    };
+    uint32_t bits = 0;
+    while ((8ull << (bits + 1)) <= (unsigned long long)a.smem_bytes / 2 && bits < 14) ++bits;
+    const uint32_t cap = lone ? 0u : 1u << bits;
+    uint32_t *key = (uint32_t *)(ohm_dsmem + room) - 2u * cap, *id = key + cap;
+    const int nsl = (R + 31) / 32;
+    uint32_t *sl = (uint32_t *)ohm_dsmem;
+    bool fail = up16(4u * (nsl + 1u)) > room - 8u * cap;
+    // widths of the 32-row slices
+    for (int s = warp; !fail && s < nsl; s += nwarps) {
+        const int li = s * 32 + lane;
+        uint32_t w = li < R ? row_len(r0 + li) : 0u;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) w = max(w, __shfl_xor_sync(0xffffffffu, w, o));
+        if (lane == 0) sl[s] = w;
     }
-    uint32_t nloc = 0;
-    const uint32_t before = block_exclusive_scan(mine, (uint32_t *)g.smem, &nloc);
-    auto up16 = [](uint32_t x) { return (x + 15u) & ~15u; };
-    const uint32_t o_rhat = up16((uint32_t)R * (uint32_t)sizeof(KRec<T>));
-    const uint32_t o_t = o_rhat + up16((uint32_t)R * (uint32_t)sizeof(T));
-    const uint32_t o_d = o_t + up16((uint32_t)R * (uint32_t)sizeof(T));
-    const uint32_t o_w = o_d + up16((uint32_t)R * (uint32_t)sizeof(T));
-    const uint32_t o_val = o_w + (wt ? up16((uint32_t)R * 8u) : 0u);
-    const uint32_t o_col = o_val + up16(nloc * (uint32_t)sizeof(T));
-    const uint32_t o_rp = o_col + up16(nloc * 4u);
-    const uint32_t o_pair = o_rp + up16((uint32_t)(R + 1) * 4u);
-    const uint32_t o_end = o_pair + up16((uint32_t)R);
-    if (o_end > (uint32_t)a.smem_bytes) return kKrylovNoSmem;      // uniform over the block
-    KRec<T> *rec = (KRec<T> *)ohm_dsmem;
-    T *rhat = (T *)(ohm_dsmem + o_rhat);
-    T *t = (T *)(ohm_dsmem + o_t);
-    T *d = (T *)(ohm_dsmem + o_d);
-    double *w = (double *)(ohm_dsmem + o_w);
-    T *lval = (T *)(ohm_dsmem + o_val);
-    uint32_t *lcol = (uint32_t *)(ohm_dsmem + o_col);
-    uint32_t *lrp = (uint32_t *)(ohm_dsmem + o_rp);
-    uint8_t *pair = ohm_dsmem + o_pair;
-    {
-        uint32_t pos = before;
-        for (int li = c0; li < c1; ++li) {
+    if (!lone) {
+        for (uint32_t q = threadIdx.x; q < cap; q += blockDim.x) key[q] = kSentinel;
+        if (threadIdx.x == 0) { s_count = 0; s_fail = 0; }
+        const uint8_t all = a.n_long > 0 ? 1 : 0;     // the chunks of a long row gather records anywhere
+        for (int i = r0 + (int)threadIdx.x; i < r1; i += blockDim.x) a.slice_export[i] = all;
+        if (!g.sync()) return false;
+        for (int li = threadIdx.x; li < R; li += blockDim.x) {
             const int i = r0 + li;
-            lrp[li] = pos;
-            if (!(a.longflag != nullptr && a.longflag[i] != 0)) {
-                for (uint32_t k = a.row_ptr[i]; k < a.row_ptr[i + 1]; ++k, ++pos) {
-                    lcol[pos] = a.col[k];
-                    lval[pos] = A[k];
+            if (pairs && a.partner[i] >= 0) a.slice_export[a.partner[i]] = 1;
+            const uint32_t k0 = a.row_ptr[i], k1 = k0 + row_len(i);
+            for (uint32_t k = k0; k < k1; ++k) {
+                const uint32_t j = a.col[k];
+                if ((int)j >= r0 && (int)j < r1) continue;
+                uint32_t pos = (j * 2654435761u) >> (32u - bits), tries = 0;
+                for (; tries < cap; ++tries, pos = (pos + 1u) & (cap - 1u)) {
+                    const uint32_t old = atomicCAS(&key[pos], kSentinel, j);
+                    if (old == j) break;
+                    if (old == kSentinel) {
+                        const int slot = atomicAdd(&s_count, 1);
+                        id[pos] = (uint32_t)slot;
+                        a.slice_export[j] = 1;
+                        if (pairs && a.partner[j] >= 0) a.slice_export[a.partner[j]] = 1;
+                        if (slot >= (int)(cap / 4u * 3u)) s_fail = 1;
+                        break;
+                    }
                 }
+                if (tries == cap) s_fail = 1;
+                if (*(volatile int *)&s_fail) break;
+            }
+            if (*(volatile int *)&s_fail) break;
+        }
+        __syncthreads();
+        m.H = s_count;
+        fail = fail || s_fail != 0;
+    } else {
+        __syncthreads();
+    }
+    // slice starts: block scan of the widths over contiguous chunks of slices
+    if (!fail) {
+        const int chunk = (nsl + (int)blockDim.x - 1) / (int)blockDim.x;
+        const int c0 = min(nsl, (int)threadIdx.x * chunk), c1 = min(nsl, c0 + chunk);
+        uint32_t mine = 0, total = 0;
+        for (int s = c0; s < c1; ++s) mine += sl[s];
+        uint32_t at = block_exclusive_scan(mine, (uint32_t *)g.smem, &total);
+        for (int s = c0; s < c1; ++s) {
+            const uint32_t w = sl[s];
+            sl[s] = at;
+            at += w;
+        }
+        if (threadIdx.x == 0) sl[nsl] = total;
+        m.W = (int)total;
+        __syncthreads();
+    }
+    const uint32_t below = room - 8u * cap;      // the table stays until the columns are known
+    const uint32_t g0 = slice_start(a.row_ptr[r0]);
+    fail = fail || R + m.H >= 0xFFFF || m.W > 0xFFFF;
+    if (!fail) {
+        const SliceOffsets chip = slice_offsets((uint32_t)R, (uint32_t)m.H, (uint32_t)m.W);
+        const SliceOffsets rest = slice_offsets((uint32_t)R, (uint32_t)m.H, 0u);
+        if (LPR == 1 && chip.end <= room && chip.z <= below) m.state = kSliceChip;
+        else if (rest.vec > room || rest.z > below || a.slice_col == nullptr) m.state = kSliceNo;
+        else if (LPR > 1) m.state = kSliceCsr;
+        else if (a.slice_val != nullptr && 32u * m.W <= slice_start(a.row_ptr[r1]) - g0) m.state = kSliceStream;
+    }
+    const SliceOffsets o = slice_offsets((uint32_t)R, (uint32_t)m.H, m.state == kSliceChip ? (uint32_t)m.W : 0u);
+    if (m.state == kSliceNo && !lone) {
+        // krylov() on this block gathers the record of every column
+        for (int i = r0 + (int)threadIdx.x; i < r1; i += blockDim.x)
+            for (uint32_t k = a.row_ptr[i]; k < a.row_ptr[i + 1]; ++k) {
+                const uint32_t j = a.col[k];
+                a.slice_export[j] = 1;
+                if (pairs && a.partner[j] >= 0) a.slice_export[a.partner[j]] = 1;
+            }
+    }
+    if (m.state != kSliceNo) {
+        uint32_t *hl = (uint32_t *)(ohm_dsmem + o.halo);
+        auto local = [&](uint32_t j) -> uint16_t {
+            if (lone || ((int)j >= r0 && (int)j < r1)) return (uint16_t)(j - (uint32_t)r0);
+            uint32_t pos = (j * 2654435761u) >> (32u - bits);
+            while (key[pos] != j) pos = (pos + 1u) & (cap - 1u);     // inserted above
+            return (uint16_t)(R + id[pos]);
+        };
+        if (m.state == kSliceCsr) {
+            for (int li = threadIdx.x; li < R; li += blockDim.x) {
+                const uint32_t k0 = a.row_ptr[r0 + li], k1 = k0 + row_len(r0 + li);
+                for (uint32_t k = k0; k < k1; ++k) a.slice_col[k] = local(a.col[k]);
             }
         }
-        if (threadIdx.x == 0) lrp[R] = nloc;
+        for (uint32_t q = threadIdx.x; q < cap; q += blockDim.x)
+            if (key[q] != kSentinel)
+                hl[id[q]] = key[q] | (pairs && a.partner[key[q]] >= 0 ? kHaloPaired : 0u);
+        if (m.state != kSliceCsr) {
+            uint16_t *lc = m.state == kSliceChip ? (uint16_t *)(ohm_dsmem + o.col) : a.slice_col + g0;
+            for (int s = warp; s < nsl; s += nwarps) {
+                const int li = s * 32 + lane;
+                const uint32_t b = sl[s], e = sl[s + 1];
+                const uint32_t k0 = li < R ? a.row_ptr[r0 + li] : 0u, len = li < R ? row_len(r0 + li) : 0u;
+                for (uint32_t k = 0; k < e - b; ++k)
+                    lc[(b + k) * 32u + lane] = k < len ? local(a.col[k0 + k]) : (uint16_t)(R + m.H);
+            }
+        }
     }
-    out.iterations = 0;
-    out.restarts = 0;
-    KRec<T> *cur = (KRec<T> *)a.rec0, *nxt = (KRec<T> *)a.rec1;
+    if (!lone && !g.sync()) return false;               // everyone's exports are marked
+    int any = 0;
+    if (m.state != kSliceNo) {
+        uint8_t *flag = ohm_dsmem + o.flag;
+        for (int li = threadIdx.x; li < R; li += blockDim.x) {
+            const int i = r0 + li;
+            uint8_t f = 0;
+            if (pairs && a.partner[i] >= 0) { f |= kRowPaired; any = 1; }
+            if (!lone && a.slice_export[i] != 0) f |= kRowExport;
+            if (a.longflag != nullptr && a.longflag[i] != 0) f |= kRowLong;
+            flag[li] = f;
+        }
+    }
+    m.pairs = __syncthreads_or(any);
+    g.map = m;
+    return true;
+}
 
-    // ---- start: r = r64, r_hat = r, p = v = d = 0; preconditioner coefficients ----
-    double acc0[2] = {0.0, 0.0};     // ||r||^2, ||W r||^2
-    for (int li = threadIdx.x; li < R; li += blockDim.x) {
-        const int i = r0 + li;
-        const T rt = cvt<T>(a.r64[i]);
-        double cs = 0.0, cp = 0.0;
-        const uint32_t ds = a.diag_slot[i];
-        const double aii = ds == kSentinel ? 0.0 : a.vals64[ds];
-        const double wi = (wt && fabs(aii) > 1e-30) ? 1.0 / fabs(aii) : 1.0;
-        if (wt) w[li] = wi;
-        const int pi = a.partner[i];
-        if (a.precond != kPcNone) {
-            if (a.precond == kPcAuto && pi >= 0) {
-                const double akk = a.diag_slot[pi] == kSentinel ? 0.0 : a.vals64[a.diag_slot[pi]];
-                const double aik = a.vals64[a.off_slot[i]];
-                const double aki = a.vals64[a.off_slot[pi]];
-                const double det = aii * akk - aik * aki;
-                if (fabs(det) > 1e-300) { cs = akk / det; cp = -aik / det; }
-            } else if (fabs(aii) > 1e-30) {
-                cs = 1.0 / aii;
-            } else if (a.precond == kPcAuto) {
-                cs = 1.0;   // unpaired zero diagonal: identity keeps M^-1 nonsingular
+// The recurrence's scalars and control, one copy per block in shared memory,
+// written by one lane of warp 0 inside the reductions (identical in every
+// block).
+enum KrylovPhase : int { kPhaseStart, kPhaseAB, kPhaseCD, kPhaseE, kPhaseDone };
+struct KrylovScalars {
+    double beta, om, al, omega;                     // read by every thread
+    double rho, rho_new, rr, rhat2, abs_tol, r0norm;
+    int phase, restart, early, code, it, restarts, flip;
+};
+
+// What follows a reduction: s holds its totals, q the scalars.
+struct KrylovLimits {
+    double tol_floor, inner_rtol;
+    int max_it, max_restarts;
+    bool accept_partial;
+};
+__device__ __forceinline__ void krylov_scalars_step(KrylovScalars &q, const double (&s)[4], const KrylovLimits &lim) {
+    bool top = false, restart = false;
+    const int phase = q.phase;
+    int code = kKrylovRunning, next = kPhaseDone;
+    if (phase == kPhaseStart) {                     // ||r||^2, ||W r||^2
+        const double r0norm = sqrt(s[1]);
+        const double abs_tol = fmax(lim.tol_floor, lim.inner_rtol * r0norm);
+        q.r0norm = r0norm;
+        q.abs_tol = abs_tol;
+        q.rr = q.rhat2 = q.rho_new = s[0];
+        q.rho = q.al = q.omega = 1.0;
+        q.it = q.restarts = 0;
+        q.early = 0;
+        q.flip = 1;                                 // toggled at the top: cur = rec0
+        if (!isfinite(r0norm)) code = kKrylovNan;
+        else if (r0norm < abs_tol || r0norm == 0.0) code = kKrylovConverged;
+        else top = true;
+    } else if (phase == kPhaseAB) {                 // (r_hat, v), ||v||^2
+        if (!(fabs(s[0]) >= kBreakdownRel * sqrt(q.rhat2 * s[1]))) {
+            if (q.restarts < lim.max_restarts && q.rr > 0.0) {
+                ++q.it;                             // cur still holds r; restart from it
+                q.flip ^= 1;
+                restart = top = true;
+            } else {
+                code = kKrylovBreakRv;
             }
         } else {
-            cs = 1.0;
+            q.al = q.rho / s[0];
+            next = kPhaseCD;
         }
-        pair[li] = pi >= 0 ? 1 : 0;
-        KRec<T> q;
-        q.p = T(0); q.v = T(0); q.r = rt; q.c = cvt<T>(cs);
-        cur[i] = q;
-        rec[li] = q;
-        ((T *)a.pc_part)[i] = cvt<T>(cp);
-        rhat[li] = rt;
-        d[li] = T(0);
-        acc0[0] += (double)rt * (double)rt;
-        acc0[1] += (wi * (double)rt) * (wi * (double)rt);
+    } else if (phase == kPhaseCD) {                 // (s,s), (t,s), (t,t), ||W s||^2
+        if (sqrt(s[3]) < q.abs_tol) {               // early exit (bicgstab.rs:134-139)
+            code = kKrylovConverged;
+            q.early = 1;
+            ++q.it;
+        } else if (!(s[2] > 0.0)) {
+            code = kKrylovBreakTt;
+        } else {
+            q.omega = s[1] / s[2];
+            next = kPhaseE;
+        }
+    } else {                                        // (r_hat, r), ||r||^2, ||W r||^2
+        const double rnorm = sqrt(s[2]);
+        q.rho_new = s[0];
+        q.rr = s[1];
+        ++q.it;
+        if (!isfinite(rnorm)) code = kKrylovNan;
+        else if (rnorm < q.abs_tol) code = kKrylovConverged;
+        else if (fabs(q.omega) < 1e-30) code = kKrylovBreakOmega;
+        else if (lim.accept_partial && q.it == lim.max_it && rnorm <= 0.5 * q.r0norm)
+            code = kKrylovConverged;                // inexact inner solve accepted
+        else top = true;
     }
-    if (!g.template allreduce<2>(acc0)) return kKrylovAbort;   // also orders the slice writes
-    const double r0norm = sqrt(acc0[1]);
-    const double abs_tol = fmax(tol_floor, inner_rtol * r0norm);
-    double rr_cur = acc0[0], rhat2 = acc0[0], rho_new = acc0[0];
-    double rho = 1.0, alpha = 1.0, omega = 1.0;
-    int code = kKrylovRunning;
-    int it = 0;
+    if (top) {
+        // top of an iteration: limit, rho breakdown test (restart with r_hat
+        // = r, p = v = 0, or stop), beta
+        q.flip ^= 1;
+        const bool stop = q.it >= lim.max_it;
+        if (!restart && !stop && !(fabs(q.rho_new) >= kBreakdownRel * sqrt(q.rhat2 * q.rr))) {
+            if (q.restarts < lim.max_restarts && q.rr > 0.0) restart = true;
+            else code = kKrylovBreakRho;
+        }
+        if (stop) code = kKrylovMaxIter;
+        if (restart) {
+            ++q.restarts;
+            q.rho = 1.0; q.al = 1.0; q.omega = 1.0;
+            q.rho_new = q.rr; q.rhat2 = q.rr;
+        }
+        if (code == kKrylovRunning) {
+            q.beta = (q.rho_new / q.rho) * (q.al / q.omega);
+            q.om = q.omega;
+            q.rho = q.rho_new;
+            next = kPhaseAB;
+        }
+    }
+    q.restart = restart ? 1 : 0;
+    q.code = code;
+    q.phase = code == kKrylovRunning ? next : kPhaseDone;
+}
 
-#define OHM_RESTART_S()                                                        \
-    do {                                                                       \
-        for (int li = threadIdx.x; li < R; li += blockDim.x) {                 \
-            KRec<T> q = rec[li];                                               \
-            q.p = T(0); q.v = T(0);                                            \
-            cur[r0 + li] = q;                                                  \
-            rec[li] = q;                                                       \
-            rhat[li] = q.r;                                                    \
-        }                                                                      \
-        OHM_SYNC_OR(kKrylovAbort);                                             \
-        rho = 1.0; alpha = 1.0; omega = 1.0;                                   \
-        rho_new = rr_cur; rhat2 = rr_cur;                                      \
-        ++out.restarts;                                                        \
-    } while (0)
+// Where the own-row vectors and the matrix slices are in the stream and csr
+// layouts, in shared memory and read again in every phase: held in registers
+// they were spilled.
+enum SliceVec : int { kVecR, kVecV, kVecP, kVecC, kVecT, kVecRhat, kVecD, kVecW, kSliceVecs };
+struct SliceView {
+    void *ptr[kSliceVecs];
+    const uint16_t *lcol;
+    void *lval;
+};
 
-    auto pc_apply = [&](int i, double c, T u, bool pr, T u_partner) -> T {
-        double z = c * (double)u;
-        if (pr) z += (double)((const T *)a.pc_part)[i] * (double)u_partner;
-        return cvt<T>(z);
+// The solve on a built slice map: a loop over phases around one reduction, so
+// that the code of an iteration stays small (written out, with a reduction
+// and a product per phase, an iteration streamed 40 KB of instructions
+// through the instruction caches, and their misses took most of it).
+template <typename T, int LPR, int MODE, class Team>
+__device__ __forceinline__ int krylov_slice(const KernelArgs &a, Team &g, double tol_floor, double inner_rtol,
+                                            int max_it, bool accept_partial, KrylovOut &out) {
+    using Acc = T;
+    __shared__ KrylovScalars S;
+    __shared__ SliceView V_;
+    const volatile SliceView &V = V_;
+    const int r0 = g.r0, r1 = g.r1, R = r1 - r0, H = g.map.H;
+    const bool pairs = g.map.pairs != 0, wt = a.newton != 0, lone = team_of_one(g), has_long = a.n_long > 0;
+    const T *A;
+    if constexpr (sizeof(T) == 4) A = (const T *)a.vals32; else A = (const T *)a.vals64;
+    const SliceOffsets o = slice_offsets((uint32_t)R, (uint32_t)H, MODE == kSliceChip ? (uint32_t)g.map.W : 0u);
+    if (threadIdx.x == 0) {
+        if constexpr (MODE != kSliceChip) {
+            // in the order of their traffic while they fit, the rest in the
+            // workspace (own rows, local index)
+            const uint32_t room = (uint32_t)a.smem_bytes & ~15u;
+            void *const spill[kSliceVecs] = {(T *)a.rself + r0, (T *)a.shat + r0, (T *)a.phat + r0,
+                                             (T *)a.cself + r0, (T *)a.t + r0,    (T *)a.rhat + r0,
+                                             (double *)a.d + r0, a.dx + r0};
+            uint32_t at = o.vec;
+            for (int k = 0; k < kSliceVecs; ++k) {
+                const bool fits = at + o.vec_bytes <= room;
+                V_.ptr[k] = fits ? (void *)(ohm_dsmem + at) : spill[k];
+                if (fits) at += o.vec_bytes;
+            }
+            const uint32_t g0 = MODE == kSliceStream ? slice_start(a.row_ptr[r0]) : 0u;
+            V_.lcol = a.slice_col + g0;
+            V_.lval = (void *)((T *)(a.slice_val + g0));
+        }
+        ((T *)(ohm_dsmem + o.z))[R + H] = T(0);          // the padding's column
+        S.phase = kPhaseStart;
+    }
+    __syncthreads();
+    // On the chip the own-row vectors are one stride apart, so a row's fields
+    // are one index and eight offsets.
+    auto vec = [&](int k) -> void * {
+        if constexpr (MODE == kSliceChip) return (void *)(ohm_dsmem + o.vec + (uint32_t)k * o.vec_bytes);
+        else return V.ptr[k];
     };
+    auto vecT = [&](int k) -> T * { return (T *)vec(k); };
+    auto zvec = [&]() -> T * { return (T *)(ohm_dsmem + o.z); };
+    auto flags = [&]() -> const uint8_t * { return ohm_dsmem + o.flag; };
+    auto lvals = [&]() -> T * {
+        if constexpr (MODE == kSliceChip) return (T *)(ohm_dsmem + o.val);
+        else return (T *)V.lval;
+    };
+    auto lcols = [&]() -> const uint16_t * {
+        if constexpr (MODE == kSliceChip) return (const uint16_t *)(ohm_dsmem + o.col);
+        else return V.lcol;
+    };
+    const KrylovLimits lim{tol_floor, inner_rtol, max_it, a.max_restarts, accept_partial};
 
-    if (!isfinite(r0norm)) {
-        code = kKrylovNan;
-    } else if (r0norm < abs_tol || r0norm == 0.0) {
-        code = kKrylovConverged;
-    } else {
-        for (; it < max_it; ++it) {
-            if (!(fabs(rho_new) >= kBreakdownRel * sqrt(rhat2 * rr_cur))) {
-                if (out.restarts < a.max_restarts && rr_cur > 0.0) {
-                    OHM_RESTART_S();
-                } else {
-                    code = kKrylovBreakRho;
-                    break;
-                }
+    for (;;) {
+        const int phase = S.phase;
+        if (phase == kPhaseDone) break;
+        double acc[4] = {0.0, 0.0, 0.0, 0.0};
+        if (phase == kPhaseE) {
+            // ---- E: d += w M^-1 s, r = s - w t; (r_hat, r), ||r||^2, ||W r||^2 ----
+            const double omega = S.omega;
+            T *r = vecT(kVecR);
+            const T *z = zvec(), *t = vecT(kVecT), *rhat = vecT(kVecRhat);
+            double *d = (double *)vec(kVecD);
+            const double *w = (const double *)vec(kVecW);
+            const uint8_t *flag = flags();
+            KRec<T> *nxt = (KRec<T> *)(S.flip ? a.rec0 : a.rec1);
+#pragma unroll 1
+            for (int li = threadIdx.x; li < R; li += blockDim.x) {
+                const T si = r[li];
+                d[li] = (double)cvt<T>(fma(omega, (double)z[li], d[li]));
+                const T rt = cvt<T>(fma(-omega, (double)t[li], (double)si));
+                r[li] = rt;
+                if (flag[li] & kRowExport) nxt[r0 + li].r = rt;
+                const double wr = wt ? w[li] * (double)rt : (double)rt;
+                acc[0] = fma((double)rhat[li], (double)rt, acc[0]);
+                acc[1] = fma((double)rt, (double)rt, acc[1]);
+                acc[2] = fma(wr, wr, acc[2]);
             }
-            const double beta = (rho_new / rho) * (alpha / omega);
-            rho = rho_new;
-            const double om = omega;
-            // ---------------- AB: p update and v = A M^-1 p ----------------
-            auto pnew = [&](const KRec<T> &q) -> T {
-                return cvt<T>(((double)q.p + (-om) * (double)q.v) * beta + (double)q.r);
-            };
-            auto phat_at = [&](int j, bool slow) -> T {
-                const KRec<T> q = cur[j];
-                double z = (double)q.c * (double)pnew(q);
-                if (slow) {
-                    const int pj = a.partner[j];
-                    if (pj >= 0) z += (double)((const T *)a.pc_part)[j] * (double)pnew(cur[pj]);
-                }
-                return cvt<T>(z);
-            };
-            double acc1[2] = {0.0, 0.0};
-            auto ab_row = [&](int i, double y) {
-                const int li = i - r0;
-                const KRec<T> q = rec[li];
-                KRec<T> n;
-                n.p = pnew(q);
-                n.v = cvt<T>(y);
-                n.r = q.r;
-                n.c = q.c;
-                nxt[i] = n;
-                rec[li] = n;
-                acc1[0] += (double)rhat[li] * (double)n.v;
-                acc1[1] += (double)n.v * (double)n.v;
-            };
-            spmv_rows<LPR, Acc, T, decltype(phat_at), decltype(ab_row), U, true>(lrp, lcol, lval, a.rowflag, r0, r1,
-                                                                            phat_at, ab_row, a.longflag, r0);
-            if (!spmv_long<Acc>(a, g, a.col, A, a.rowflag, phat_at, ab_row)) return kKrylovAbort;
-            if (!g.template allreduce<2>(acc1)) return kKrylovAbort;
-            if (!(fabs(acc1[0]) >= kBreakdownRel * sqrt(rhat2 * acc1[1]))) {
-                if (out.restarts < a.max_restarts && rr_cur > 0.0) {
-                    OHM_RESTART_S();
-                    continue;
-                }
-                code = kKrylovBreakRv;
-                break;
-            }
-            alpha = rho / acc1[0];
-            const double al = alpha;
-            // ---------------- CD: s = r - a v and t = A M^-1 s ----------------
-            auto s_of = [&](const KRec<T> &q) -> T {
-                return cvt<T>((double)q.r + (-al) * (double)q.v);
-            };
-            // After AB every own row's record is the same in shared memory and
-            // in nxt, and CD rewrites neither: columns of this block are
-            // gathered from shared memory (the same values, no L2 round trip).
-            auto rec_at = [&](int j) -> KRec<T> {
-                return (unsigned)(j - r0) < (unsigned)R ? rec[j - r0] : nxt[j];
-            };
-            auto shat_at = [&](int j, bool slow) -> T {
-                const KRec<T> q = rec_at(j);
-                double z = (double)q.c * (double)s_of(q);
-                if (slow) {
-                    const int pj = a.partner[j];
-                    if (pj >= 0) z += (double)((const T *)a.pc_part)[j] * (double)s_of(rec_at(pj));
-                }
-                return cvt<T>(z);
-            };
-            double acc3[4] = {0.0, 0.0, 0.0, 0.0};   // (s,s), (t,s), (t,t), ||W s||^2
-            auto cd_row = [&](int i, double y) {
-                const int li = i - r0;
-                const T si = s_of(rec[li]);
-                const T ti = cvt<T>(y);
-                t[li] = ti;
-                if (pair[li]) ((T *)a.s)[i] = si;
-                const double ws = wt ? w[li] * (double)si : (double)si;
-                acc3[0] += (double)si * (double)si;
-                acc3[1] += (double)ti * (double)si;
-                acc3[2] += (double)ti * (double)ti;
-                acc3[3] += ws * ws;
-            };
-            spmv_rows<LPR, Acc, T, decltype(shat_at), decltype(cd_row), U, true>(lrp, lcol, lval, a.rowflag, r0, r1,
-                                                                            shat_at, cd_row, a.longflag, r0);
-            if (!spmv_long<Acc>(a, g, a.col, A, a.rowflag, shat_at, cd_row)) return kKrylovAbort;
-            if (!g.template allreduce<4>(acc3)) return kKrylovAbort;
-            if (sqrt(acc3[3]) < abs_tol) {          // early exit (bicgstab.rs:134-139)
+        } else if (phase != kPhaseStart) {
+            // ---- AB: p update, v = A M^-1 p; (r_hat, v), ||v||^2 ----
+            // ---- CD: s = r - a v (kept in r), d += a M^-1 p, t = A M^-1 s;
+            //      (s, s), (t, s), (t, t), ||W s||^2 ----
+            const bool cd = phase == kPhaseCD;
+            KRec<T> *cur = (KRec<T> *)(S.flip ? a.rec1 : a.rec0), *nxt = (KRec<T> *)(S.flip ? a.rec0 : a.rec1);
+            if (!cd && S.restart) {
+                const uint8_t *flag = flags();
+                T *p = vecT(kVecP), *v = vecT(kVecV), *r = vecT(kVecR), *c = vecT(kVecC), *rhat = vecT(kVecRhat);
+#pragma unroll 1
                 for (int li = threadIdx.x; li < R; li += blockDim.x) {
-                    const int i = r0 + li;
-                    const KRec<T> q = rec[li];
-                    const bool pr = pair[li] != 0;
-                    const T ph = pc_apply(i, (double)q.c, q.p, pr, pr ? nxt[a.partner[i]].p : T(0));
-                    d[li] = cvt<T>((double)d[li] + al * (double)ph);
+                    p[li] = T(0);
+                    v[li] = T(0);
+                    rhat[li] = r[li];
+                    if (flag[li] & kRowExport) cur[r0 + li] = KRec<T>{T(0), T(0), r[li], c[li]};
                 }
-                code = kKrylovConverged;
-                ++it;
-                break;
+                OHM_SYNC_OR(kKrylovAbort);
             }
-            if (!(acc3[2] > 0.0)) { code = kKrylovBreakTt; break; }
-            omega = acc3[1] / acc3[2];
-            // ---------------- E: d, r updates ----------------
-            double acc4[3] = {0.0, 0.0, 0.0};   // (r_hat, r), ||r||^2, ||W r||^2
+            // the vector that M^-1 is applied to: p's update or s
+            const double kv = cd ? -S.al : -S.om, beta = S.beta;
+            auto u3 = [&](T pp, T vv, T rr) -> T {
+                const double base = cd ? (double)rr : (double)pp;
+                const double x = fma(kv, (double)vv, base);
+                return cvt<T>(cd ? x : fma(x, beta, (double)rr));
+            };
+            auto u = [&](const KRec<T> &q) -> T { return u3(q.p, q.v, q.r); };
+            const KRec<T> *buf = cd ? nxt : cur;
+            T *const up = cd ? vecT(kVecR) : vecT(kVecP);        // where the own rows of it are kept
+            {
+                // z of the halo rows from their published records; the first
+                // one is fetched before the own rows' work, so its round trip
+                // overlaps it
+                const uint32_t *hl = (const uint32_t *)(ohm_dsmem + o.halo);
+                T *z = zvec();
+                int h = threadIdx.x;
+                uint32_t e = 0;
+                KRec<T> q{};
+                if (h < H) {
+                    e = hl[h];
+                    q = buf[e & ~kHaloPaired];
+                }
+                {
+                    const T *p = vecT(kVecP), *v = vecT(kVecV), *r = vecT(kVecR), *c = vecT(kVecC);
+                    double *d = (double *)vec(kVecD);
+                    const double al = S.al;
+#pragma unroll 1
+                    for (int li = threadIdx.x; li < R; li += blockDim.x) {
+                        const T un = u3(p[li], v[li], r[li]);
+                        if (cd) d[li] = fma(al, (double)z[li], d[li]);
+                        up[li] = un;
+                        z[li] = cvt<T>((double)c[li] * (double)un);
+                    }
+                }
+                while (h < H) {
+                    double zz = (double)q.c * (double)u(q);
+                    if (e & kHaloPaired) {
+                        const uint32_t j = e & ~kHaloPaired;
+                        zz = fma((double)((const T *)a.pc_part)[j], (double)u(buf[a.partner[j]]), zz);
+                    }
+                    z[R + h] = cvt<T>(zz);
+                    h += blockDim.x;
+                    if (h >= H) break;
+                    e = hl[h];
+                    q = buf[e & ~kHaloPaired];
+                }
+            }
+            if (pairs) {
+                // own paired rows: the partner's term
+                __syncthreads();
+                const uint8_t *flag = flags();
+                const T *c = vecT(kVecC);
+                T *z = zvec();
+#pragma unroll 1
+                for (int li = threadIdx.x; li < R; li += blockDim.x) {
+                    if (!(flag[li] & kRowPaired)) continue;
+                    const int pi = a.partner[r0 + li];
+                    const T other = (pi >= r0 && pi < r1) ? up[pi - r0] : u(buf[pi]);
+                    double zz = (double)c[li] * (double)up[li];
+                    zz = fma((double)((const T *)a.pc_part)[r0 + li], (double)other, zz);
+                    z[li] = cvt<T>(zz);
+                    if (cd && !lone) ((T *)a.s)[r0 + li] = up[li];
+                }
+            }
+            __syncthreads();
+            // y = A z on the own rows
+            const uint8_t *flag = flags();
+            auto row = [&](int i, double y) {
+                const int li = i - r0;
+                const T yt = cvt<T>(y), ui = up[li];
+                if (cd) {
+                    vecT(kVecT)[li] = yt;
+                    const double ws = wt ? ((const double *)vec(kVecW))[li] * (double)ui : (double)ui;
+                    acc[0] = fma((double)ui, (double)ui, acc[0]);
+                    acc[1] = fma((double)yt, (double)ui, acc[1]);
+                    acc[2] = fma((double)yt, (double)yt, acc[2]);
+                    acc[3] = fma(ws, ws, acc[3]);
+                } else {
+                    vecT(kVecV)[li] = yt;
+                    if (flag[li] & kRowExport) nxt[i] = KRec<T>{ui, yt, vecT(kVecR)[li], vecT(kVecC)[li]};
+                    acc[0] = fma((double)vecT(kVecRhat)[li], (double)yt, acc[0]);
+                    acc[1] = fma((double)yt, (double)yt, acc[1]);
+                }
+            };
+            if constexpr (MODE == kSliceCsr) {
+                const T *z = zvec();
+                auto zx = [&](int j, bool) -> T { return z[j]; };
+                spmv_rows<LPR, Acc, T, decltype(zx), decltype(row), kRowsInFlight, false>(
+                    a.row_ptr, lcols(), A, (const uint8_t *)nullptr, r0, r1, zx, row, a.longflag);
+            } else {
+                const int lane = threadIdx.x & 31;
+                const uint32_t *sl = (const uint32_t *)ohm_dsmem;
+                const T *z = zvec(), *lval = lvals();
+                const uint16_t *lcol = lcols();
+#pragma unroll 1
+                for (int li = threadIdx.x; li - lane < R; li += blockDim.x) {
+                    const int s = li >> 5;
+                    const uint32_t e = sl[s + 1] * 32u;
+                    uint32_t k = sl[s] * 32u + lane;
+                    Acc y = Acc(0);
+#pragma unroll 1
+                    for (; k + 96u < e; k += 128u) {
+                        const T z0 = z[lcol[k]], z1 = z[lcol[k + 32u]], z2 = z[lcol[k + 64u]], z3 = z[lcol[k + 96u]];
+                        y += (Acc)lval[k] * (Acc)z0;
+                        y += (Acc)lval[k + 32u] * (Acc)z1;
+                        y += (Acc)lval[k + 64u] * (Acc)z2;
+                        y += (Acc)lval[k + 96u] * (Acc)z3;
+                    }
+#pragma unroll 1
+                    for (; k < e; k += 32u) y += (Acc)lval[k] * (Acc)z[lcol[k]];
+                    if (li < R && !(has_long && (flag[li] & kRowLong))) row(r0 + li, (double)y);
+                }
+            }
+            if (has_long) {
+                auto z_at = [&](int j, bool slow) -> T {
+                    const KRec<T> q = buf[j];
+                    double zz = (double)q.c * (double)u(q);
+                    if (slow) {
+                        const int pj = a.partner[j];
+                        if (pj >= 0) zz = fma((double)((const T *)a.pc_part)[j], (double)u(buf[pj]), zz);
+                    }
+                    return cvt<T>(zz);
+                };
+                if (!spmv_long<Acc>(a, g, a.col, A, a.rowflag, z_at, row)) return kKrylovAbort;
+            }
+        } else {
+            // ---- start: matrix slices' values, r = r64, r_hat = r, p = v =
+            //      d = 0, preconditioner coefficients; ||r||^2, ||W r||^2 ----
+            const uint8_t *flag = flags();
+            if constexpr (MODE != kSliceCsr) {
+                const int lane = threadIdx.x & 31;
+                const uint32_t *sl = (const uint32_t *)ohm_dsmem;
+                T *lval = lvals();
+#pragma unroll 1
+                for (int li = threadIdx.x; li - lane < R; li += blockDim.x) {
+                    const int s = li >> 5;
+                    const uint32_t b = sl[s], width = sl[s + 1] - b;
+                    uint32_t k0 = 0, len = 0;
+                    if (li < R && !(flag[li] & kRowLong)) {
+                        k0 = a.row_ptr[r0 + li];
+                        len = a.row_ptr[r0 + li + 1] - k0;
+                    }
+#pragma unroll 4
+                    for (uint32_t k = 0; k < width; ++k) lval[(b + k) * 32u + lane] = k < len ? A[k0 + k] : T(0);
+                }
+            }
+            T *p = vecT(kVecP), *v = vecT(kVecV), *r = vecT(kVecR), *c = vecT(kVecC), *rhat = vecT(kVecRhat);
+            double *d = (double *)vec(kVecD), *w = (double *)vec(kVecW);
+#pragma unroll 1
             for (int li = threadIdx.x; li < R; li += blockDim.x) {
                 const int i = r0 + li;
-                const KRec<T> q = rec[li];
-                const bool pr = pair[li] != 0;
-                const int pi = pr ? a.partner[i] : i;
-                const T ph = pc_apply(i, (double)q.c, q.p, pr, pr ? nxt[pi].p : T(0));
-                const T si = s_of(q);
-                const T sh = pc_apply(i, (double)q.c, si, pr, pr ? ((const T *)a.s)[pi] : T(0));
-                d[li] = cvt<T>(((double)d[li] + al * (double)ph) + omega * (double)sh);
-                const T rt = cvt<T>((double)si + (-omega) * (double)t[li]);
-                nxt[i].r = rt;
-                rec[li].r = rt;
-                const double wr = wt ? w[li] * (double)rt : (double)rt;
-                acc4[0] += (double)rhat[li] * (double)rt;
-                acc4[1] += (double)rt * (double)rt;
-                acc4[2] += wr * wr;
-            }
-            if (!g.template allreduce<3>(acc4)) return kKrylovAbort;
-            { KRec<T> *tmp = cur; cur = nxt; nxt = tmp; }
-            rho_new = acc4[0];
-            rr_cur = acc4[1];
-            const double rnorm = sqrt(acc4[2]);
-            if (!isfinite(rnorm)) { code = kKrylovNan; ++it; break; }
-            if (rnorm < abs_tol) { code = kKrylovConverged; ++it; break; }
-            if (fabs(omega) < 1e-30) { code = kKrylovBreakOmega; ++it; break; }
-            if (accept_partial && it + 1 == max_it && rnorm <= 0.5 * r0norm) {
-                code = kKrylovConverged;
-                ++it;
-                break;
+                const T rt = cvt<T>(a.r64[i]);
+                double cs = 0.0, cp = 0.0;
+                const uint32_t ds = a.diag_slot[i];
+                const double aii = ds == kSentinel ? 0.0 : a.vals64[ds];
+                const double wi = (wt && fabs(aii) > 1e-30) ? 1.0 / fabs(aii) : 1.0;
+                if (wt) w[li] = wi;
+                if (a.precond != kPcNone) {
+                    if (flag[li] & kRowPaired) {
+                        const int pi = a.partner[i];
+                        const double akk = a.diag_slot[pi] == kSentinel ? 0.0 : a.vals64[a.diag_slot[pi]];
+                        const double aik = a.vals64[a.off_slot[i]];
+                        const double aki = a.vals64[a.off_slot[pi]];
+                        const double det = aii * akk - aik * aki;
+                        if (fabs(det) > 1e-300) { cs = akk / det; cp = -aik / det; }
+                        ((T *)a.pc_part)[i] = cvt<T>(cp);
+                    } else if (fabs(aii) > 1e-30) {
+                        cs = 1.0 / aii;
+                    } else if (a.precond == kPcAuto) {
+                        cs = 1.0;   // unpaired zero diagonal: identity keeps M^-1 nonsingular
+                    }
+                } else {
+                    cs = 1.0;
+                }
+                p[li] = T(0);
+                v[li] = T(0);
+                r[li] = rt;
+                c[li] = cvt<T>(cs);
+                rhat[li] = rt;
+                d[li] = 0.0;
+                if (flag[li] & kRowExport) ((KRec<T> *)a.rec0)[i] = KRec<T>{T(0), T(0), rt, cvt<T>(cs)};
+                acc[0] = fma((double)rt, (double)rt, acc[0]);
+                acc[1] = fma(wi * (double)rt, wi * (double)rt, acc[1]);
             }
         }
-        if (code == kKrylovRunning) code = kKrylovMaxIter;
+        if (!g.template reduce_then<4>(acc, [&](const double (&s)[4], bool writer) {
+                if (writer) krylov_scalars_step(S, s, lim);
+            }))
+            return kKrylovAbort;
     }
-#undef OHM_RESTART_S
-    out.iterations = it;
-    if (code == kKrylovConverged)
-        for (int li = threadIdx.x; li < R; li += blockDim.x) a.dx[r0 + li] = (double)d[li];
+    const int code = S.code;
+    if (code == kKrylovConverged) {
+        // an early exit left d + a M^-1 p unrounded
+        const bool early = S.early != 0;
+        const double *d = (const double *)vec(kVecD);
+#pragma unroll 1
+        for (int li = threadIdx.x; li < R; li += blockDim.x)
+            a.dx[r0 + li] = early ? (double)cvt<T>(d[li]) : d[li];
+    }
+    out.iterations = S.it;
+    out.restarts = S.restarts;
+    __syncthreads();                                   // S is rewritten by the next solve
     return code;
 }
 
@@ -974,10 +1386,14 @@ template <typename T, int LPR, class Team>
 __device__ __forceinline__ int krylov_any(const KernelArgs &a, Team &g, double tol_floor, double inner_rtol,
                                           int max_it, bool accept_partial, KrylovOut &out) {
     if (a.precond == kPcIsai) return krylov_isai<T, LPR>(a, g, tol_floor, inner_rtol, max_it, accept_partial, out);
-    if constexpr (std::is_same<Team, GridTeam>::value) {
-        const int code = krylov_smem<T, LPR, (LPR == 1 ? 2 : 4)>(a, g, tol_floor, inner_rtol, max_it,
-                                                                 accept_partial, out);
-        if (code != kKrylovNoSmem) return code;
+    if (g.map.state == kSliceNone && !slice_map<LPR>(a, g)) return kKrylovAbort;
+    if constexpr (LPR == 1) {
+        if (g.map.state == kSliceChip)
+            return krylov_slice<T, LPR, kSliceChip>(a, g, tol_floor, inner_rtol, max_it, accept_partial, out);
+        if (g.map.state == kSliceStream)
+            return krylov_slice<T, LPR, kSliceStream>(a, g, tol_floor, inner_rtol, max_it, accept_partial, out);
+    } else if (g.map.state == kSliceCsr) {
+        return krylov_slice<T, LPR, kSliceCsr>(a, g, tol_floor, inner_rtol, max_it, accept_partial, out);
     }
     return krylov<T, LPR>(a, g, tol_floor, inner_rtol, max_it, accept_partial, out);
 }
@@ -1199,19 +1615,16 @@ __device__ __forceinline__ bool newton_run(const KernelArgs &a, Team &g, const R
         }
         KrylovOut ko{0, 0};
         int it32 = 0, it64 = 0;
+        bool run64 = true;
         if (a.mixed && !(a.newton && eta < a.fp32_min_eta)) {
             kcode = krylov_any<float, LPR>(a, g, floor_tol, eta, min(a.fp32_max_iterations, cfg.max_krylov), true, ko);
             if (kcode == kKrylovAbort) return false;
             it32 = ko.iterations;
             restarts += ko.restarts;
-            if (kcode != kKrylovConverged) {
-                ++fallbacks;           // FP32 failed or stalled: redo this solve in FP64
-                kcode = krylov_any<double, LPR>(a, g, floor_tol, eta, cfg.max_krylov, false, ko);
-                if (kcode == kKrylovAbort) return false;
-                it64 = ko.iterations;
-                restarts += ko.restarts;
-            }
-        } else {
+            run64 = kcode != kKrylovConverged;
+            if (run64) ++fallbacks;    // FP32 failed or stalled: redo this solve in FP64
+        }
+        if (run64) {
             kcode = krylov_any<double, LPR>(a, g, floor_tol, eta, cfg.max_krylov, false, ko);
             if (kcode == kKrylovAbort) return false;
             it64 = ko.iterations;
@@ -1466,20 +1879,9 @@ __device__ __forceinline__ bool solve_body(const KernelArgs &a, Team &g, DeviceI
 
 // One large system per launch: the whole (co-resident) grid is the team.
 template <int LPR>
-__global__ void __launch_bounds__(kSolverBlock, 1) persistent_solver(KernelArgs a) {
-    __shared__ double smem[32 * 4 + 4];   // GridTeam reductions: warp values + results
+__global__ void __launch_bounds__(kSolverBlock, 1) persistent_solver(const __grid_constant__ KernelArgs a) {
     GridTeam g;
-    g.G = gridDim.x;
-    g.bid = blockIdx.x;
-    g.r0 = (int)(((long long)a.n * g.bid) / g.G);
-    g.r1 = (int)(((long long)a.n * (g.bid + 1)) / g.G);
-    g.gtid = g.bid * blockDim.x + threadIdx.x;
-    g.gstride = g.G * blockDim.x;
-    g.smem = smem;
-    g.partials = a.partials;
-    g.red = 0;
-    g.epoch = 0;
-    g.gs = a.gs;
+    g.init(a);
     solve_body<LPR>(a, g, a.info);
 }
 

@@ -1,0 +1,9 @@
+// Adaptive transient kernel, 8 lane(s) per row.
+#include "transient_kernel.cuh"
+
+namespace ohm {
+
+template <>
+AdaptFn adaptive_kernel_for<8>() { return adaptive_kernel<8>; }
+
+}  // namespace ohm

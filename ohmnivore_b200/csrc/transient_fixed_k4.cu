@@ -1,0 +1,9 @@
+// Fixed-step transient kernel, 4 lane(s) per row.
+#include "transient_kernel.cuh"
+
+namespace ohm {
+
+template <>
+TranFn transient_kernel_for<4>() { return transient_kernel<4>; }
+
+}  // namespace ohm

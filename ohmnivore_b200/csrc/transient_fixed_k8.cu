@@ -1,0 +1,9 @@
+// Fixed-step transient kernel, 8 lane(s) per row.
+#include "transient_kernel.cuh"
+
+namespace ohm {
+
+template <>
+TranFn transient_kernel_for<8>() { return transient_kernel<8>; }
+
+}  // namespace ohm
