@@ -285,6 +285,31 @@ static ohm_status batch_args(ohm_batch *b, double *x_dev, const ohm_newton_param
     return OHM_OK;
 }
 
+// Dynamic shared memory of a block: an equal share of an SM's, less where the
+// largest circuit needs less.  A circuit whose slice does not fit keeps its
+// gather vector and as many of its vectors there as do (krylov_slice()).
+static int batch_smem_bytes(ohm_batch *b, BatchFn fn, int shape) {
+    int dev = 0, sm_total = 0, optin = 0;
+    cudaFuncAttributes fa{};
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sm_total, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+        cudaFuncGetAttributes(&fa, (const void *)fn) != cudaSuccess)
+        return 0;
+    const int64_t share = std::min<int64_t>(optin, sm_total / kBatchShapes[shape].min_blocks - 1024) -
+                          (int64_t)fa.sharedSizeBytes;
+    int64_t need = 0;
+    for (const InstanceOffsets &o : b->h_offsets) {
+        const int64_t n = o.ro1 - o.ro, z = o.no1 - o.no;
+        need = std::max(need, n * (9 * 8 + 1) + n / 8 + (z + z / 4) * (8 + 2) + 512);
+    }
+    const int64_t bytes = std::min(share, need) & ~(int64_t)15;
+    if (bytes <= 0 || cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)bytes) != cudaSuccess)
+        return 0;
+    return (int)bytes;
+}
+
 // One launch over `n` instances listed in `order` (device): a persistent grid
 // of (blocks per SM) x SMs blocks, each taking instances from the queue.
 static ohm_status launch_batch(ohm_batch *b, BatchArgs B, int lpr, int shape, int n, const int32_t *order) {
@@ -293,12 +318,13 @@ static ohm_status launch_batch(ohm_batch *b, BatchArgs B, int lpr, int shape, in
     B.n_inst = n;
     BatchFn fn = batch_kernel(lpr, shape);
     const int block = kBatchShapes[shape].block;
+    B.base.smem_bytes = batch_smem_bytes(b, fn, shape);
     int per_sm = 0;
-    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, block, 0));
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, block, B.base.smem_bytes));
     if (per_sm < 1) return ohm_fail(OHM_ERR_CUDA, "batch kernel does not fit on an SM");
     const int grid = (int)std::min<int64_t>((int64_t)per_sm * c->num_sms, n);
     CUDA_TRY(cudaMemsetAsync(b->queue, 0, sizeof(unsigned int), c->stream));
-    fn<<<grid, block, 0, c->stream>>>(B);
+    fn<<<grid, block, B.base.smem_bytes, c->stream>>>(B);
     CUDA_TRY(cudaGetLastError());
     return OHM_OK;
 }

@@ -210,8 +210,8 @@ __device__ __forceinline__ bool grid_barrier(const GridSync &gs) {
 // j + 1 while a slower one still reads reduction j, never j + 2.  Returns
 // false when a barrier wait gave up.
 template <int NV, bool MAX, typename Fin>
-__device__ __forceinline__ bool team_reduce_then(int G, bool cluster, double *partials, const GridSync &gs,
-                                                 const double (&v)[NV], Fin fin) {
+__device__ __forceinline__ bool team_reduce_then(int G, int rank, bool cluster, double *partials,
+                                                 const GridSync &gs, const double (&v)[NV], Fin fin) {
     ReduceBuffers &buf = reduce_buffers();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nwarps = (blockDim.x + 31) >> 5;
@@ -224,7 +224,7 @@ __device__ __forceinline__ bool team_reduce_then(int G, bool cluster, double *pa
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) y = combine2<MAX>(y, __shfl_xor_sync(0xffffffffu, y, o));
             if (lane < G) {
-                const uint32_t local = (uint32_t)__cvta_generic_to_shared(buf.box + half * 64 + warp * 16 + blockIdx.x);
+                const uint32_t local = (uint32_t)__cvta_generic_to_shared(buf.box + half * 64 + warp * 16 + rank);
                 uint32_t remote;
                 asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(lane));
                 asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(remote), "d"(y) : "memory");
@@ -245,7 +245,7 @@ __device__ __forceinline__ bool team_reduce_then(int G, bool cluster, double *pa
                 double *p = partials + (size_t)half * 4 * G;
                 const double x = warp_totals<NV, MAX>(w, lane);
                 const int kv = warp_value<NV>(lane);
-                if (lane % kWarpValueLanes<NV> == 0 && kv < NV) p[kv * G + blockIdx.x] = x;
+                if (lane % kWarpValueLanes<NV> == 0 && kv < NV) p[kv * G + rank] = x;
                 __syncwarp();
                 if (lane == 0) {
                     const unsigned long long e = buf.epoch + (unsigned)G;

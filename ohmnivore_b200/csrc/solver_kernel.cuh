@@ -258,7 +258,7 @@ struct GridTeam {
     __device__ __forceinline__ bool leader() const { return blockIdx.x == 0 && threadIdx.x == 0; }
     template <int NV, bool MAX = false, typename Fin>
     __device__ __forceinline__ bool reduce_then(const double (&v)[NV], Fin fin) {
-        return team_reduce_then<NV, MAX>((int)gridDim.x, cluster, partials, gs, v, fin);
+        return team_reduce_then<NV, MAX>((int)gridDim.x, (int)blockIdx.x, cluster, partials, gs, v, fin);
     }
     template <int NV, bool MAX>
     __device__ __forceinline__ bool reduce(double (&v)[NV]) {
@@ -286,7 +286,7 @@ struct BlockTeam {
 
     template <int NV, bool MAX = false, typename Fin>
     __device__ __forceinline__ bool reduce_then(const double (&v)[NV], Fin fin) {
-        return team_reduce_then<NV, MAX>(1, false, nullptr, GridSync{nullptr, nullptr}, v, fin);
+        return team_reduce_then<NV, MAX>(1, 0, false, nullptr, GridSync{nullptr, nullptr}, v, fin);
     }
 
     __device__ __forceinline__ bool sync() { __syncthreads(); return true; }
@@ -975,9 +975,22 @@ __device__ __forceinline__ bool slice_map(const KernelArgs &a, Team &g) {
 enum KrylovPhase : int { kPhaseStart, kPhaseAB, kPhaseCD, kPhaseE, kPhaseDone };
 struct KrylovScalars {
     double beta, om, al, omega;                     // read by every thread
-    double rho, rho_new, rr, rhat2, abs_tol, r0norm;
+    double rho, rho_new, rr, rhat2, abs_tol, r0norm, tol2;
     int phase, restart, early, code, it, restarts, flip;
 };
+
+// |x| < rel sqrt(y), compared as squares: a square root is 120 cycles on the
+// one lane that every thread waits for.  Where a square would leave the
+// normal range the root decides.
+__device__ __forceinline__ bool below_root(double x, double rel, double y) {
+    const double x2 = x * x, y2 = rel * rel * y;
+    if (x2 > 1e-290 && x2 < 1e290 && y2 > 1e-290 && y2 < 1e290) return x2 < y2;
+    return !(fabs(x) >= rel * sqrt(y));
+}
+// sqrt(y) < tol, tol2 = tol^2.
+__device__ __forceinline__ bool root_below(double y, double tol, double tol2) {
+    return tol2 > 1e-290 && tol2 < 1e290 ? y < tol2 : sqrt(y) < tol;
+}
 
 // What follows a reduction: s holds its totals, q the scalars.
 struct KrylovLimits {
@@ -994,6 +1007,7 @@ __device__ __forceinline__ void krylov_scalars_step(KrylovScalars &q, const doub
         const double abs_tol = fmax(lim.tol_floor, lim.inner_rtol * r0norm);
         q.r0norm = r0norm;
         q.abs_tol = abs_tol;
+        q.tol2 = abs_tol * abs_tol;
         q.rr = q.rhat2 = q.rho_new = s[0];
         q.rho = q.al = q.omega = 1.0;
         q.it = q.restarts = 0;
@@ -1003,7 +1017,7 @@ __device__ __forceinline__ void krylov_scalars_step(KrylovScalars &q, const doub
         else if (r0norm < abs_tol || r0norm == 0.0) code = kKrylovConverged;
         else top = true;
     } else if (phase == kPhaseAB) {                 // (r_hat, v), ||v||^2
-        if (!(fabs(s[0]) >= kBreakdownRel * sqrt(q.rhat2 * s[1]))) {
+        if (below_root(s[0], kBreakdownRel, q.rhat2 * s[1])) {
             if (q.restarts < lim.max_restarts && q.rr > 0.0) {
                 ++q.it;                             // cur still holds r; restart from it
                 q.flip ^= 1;
@@ -1016,7 +1030,7 @@ __device__ __forceinline__ void krylov_scalars_step(KrylovScalars &q, const doub
             next = kPhaseCD;
         }
     } else if (phase == kPhaseCD) {                 // (s,s), (t,s), (t,t), ||W s||^2
-        if (sqrt(s[3]) < q.abs_tol) {               // early exit (bicgstab.rs:134-139)
+        if (root_below(s[3], q.abs_tol, q.tol2)) {  // early exit (bicgstab.rs:134-139)
             code = kKrylovConverged;
             q.early = 1;
             ++q.it;
@@ -1027,14 +1041,13 @@ __device__ __forceinline__ void krylov_scalars_step(KrylovScalars &q, const doub
             next = kPhaseE;
         }
     } else {                                        // (r_hat, r), ||r||^2, ||W r||^2
-        const double rnorm = sqrt(s[2]);
         q.rho_new = s[0];
         q.rr = s[1];
         ++q.it;
-        if (!isfinite(rnorm)) code = kKrylovNan;
-        else if (rnorm < q.abs_tol) code = kKrylovConverged;
+        if (!isfinite(s[2])) code = kKrylovNan;
+        else if (root_below(s[2], q.abs_tol, q.tol2)) code = kKrylovConverged;
         else if (fabs(q.omega) < 1e-30) code = kKrylovBreakOmega;
-        else if (lim.accept_partial && q.it == lim.max_it && rnorm <= 0.5 * q.r0norm)
+        else if (lim.accept_partial && q.it == lim.max_it && sqrt(s[2]) <= 0.5 * q.r0norm)
             code = kKrylovConverged;                // inexact inner solve accepted
         else top = true;
     }
@@ -1043,7 +1056,7 @@ __device__ __forceinline__ void krylov_scalars_step(KrylovScalars &q, const doub
         // = r, p = v = 0, or stop), beta
         q.flip ^= 1;
         const bool stop = q.it >= lim.max_it;
-        if (!restart && !stop && !(fabs(q.rho_new) >= kBreakdownRel * sqrt(q.rhat2 * q.rr))) {
+        if (!restart && !stop && below_root(q.rho_new, kBreakdownRel, q.rhat2 * q.rr)) {
             if (q.restarts < lim.max_restarts && q.rr > 0.0) restart = true;
             else code = kKrylovBreakRho;
         }
