@@ -1,8 +1,9 @@
 // AC sweep: A(f) x(f) = b_ac with A(f) = G + j 2 pi f C for many frequency
 // points in one launch (src/analysis/ac.rs:56-70 solves them one at a time).
 //
-// One thread block per frequency point, taken from a work queue; each runs a
-// complex FP64 right-preconditioned BiCGSTAB with the reference's operation
+// One thread-block cluster per frequency point where its shared memory holds
+// the point, else one thread block per point (or a team of them), taken from
+// a work queue; each runs a complex FP64 right-preconditioned BiCGSTAB with the reference's operation
 // order (src/solver/gpu.rs:608-690: conjugated dots sum(conj(x) y), stop at
 // ||r|| < tol ||b||).  A(f) is never stored: the SpMV reads the shared G and
 // C values of one pattern and forms g + j w c per nonzero, so every
@@ -39,7 +40,8 @@ struct AcArgs {
     const double *omega;               // per frequency point of this launch
     const int32_t *partner;
     const uint32_t *diag_slot, *off_slot;
-    double2 *work;                     // kAcVecs * n per frequency point
+    double2 *work;                     // vecs * n per frequency point
+    int vecs;
     AcDev *info;
     unsigned int *queue;
     // Team mode (fewer points than resident blocks): block b works on point
@@ -127,6 +129,34 @@ __device__ __forceinline__ double2 cval(const AcArgs &A, uint32_t k, double w) {
     return make_double2(A.g[k], A.c ? w * A.c[k] : 0.0);
 }
 
+// Block-Jacobi coefficients of row i at this frequency: the row's own
+// (returned) and its partner's (cp).
+__device__ __forceinline__ double2 ac_precond(const AcArgs &A, int i, double w, double2 &cp) {
+    double2 cs = make_double2(0.0, 0.0);
+    cp = make_double2(0.0, 0.0);
+    const uint32_t ds = A.diag_slot[i];
+    const double2 aii = ds == kSentinel ? make_double2(0.0, 0.0) : cval(A, ds, w);
+    const int pi = A.partner[i];
+    if (A.precond == kPcNone) {
+        cs = make_double2(1.0, 0.0);
+    } else if (A.precond == kPcAuto && pi >= 0) {
+        // [[a_ii a_ik] [a_ki a_kk]]^-1, the row-i half
+        const uint32_t dk = A.diag_slot[pi];
+        const double2 akk = dk == kSentinel ? make_double2(0.0, 0.0) : cval(A, dk, w);
+        const double2 aik = cval(A, A.off_slot[i], w), aki = cval(A, A.off_slot[pi], w);
+        const double2 det = csub(cmul(aii, akk), cmul(aik, aki));
+        if (cabs2(det) > 1e-300) {
+            cs = cdiv(akk, det);
+            cp = cdiv(make_double2(-aik.x, -aik.y), det);
+        }
+    } else if (cabs2(aii) > 1e-30) {
+        cs = cdiv(make_double2(1.0, 0.0), aii);        // gpu.rs:300-313
+    } else if (A.precond == kPcAuto) {
+        cs = make_double2(1.0, 0.0);
+    }
+    return cs;
+}
+
 // y_i = sum_k A(f)_ik x_k for rows [r0, r1), LPR lanes per row; f(i, y).
 template <int LPR, typename F>
 __device__ __forceinline__ void cspmv(const AcArgs &A, double w, const double2 *x, int r0, int r1, F f) {
@@ -159,7 +189,7 @@ __device__ bool ac_point(const AcArgs &A, int q, AcTeam<TEAM> &g) {
     const int n = A.n, r0 = g.r0, r1 = g.r1;
     {
         const double w = A.omega[q];
-        double2 *W = A.work + (size_t)q * kAcVecs * n;
+        double2 *W = A.work + (size_t)q * A.vecs * n;
         double2 *x = W, *r = W + n, *rh = W + 2 * (size_t)n, *p = W + 3 * (size_t)n, *v = W + 4 * (size_t)n;
         double2 *s = W + 5 * (size_t)n, *t = W + 6 * (size_t)n, *ph = W + 7 * (size_t)n, *sh = W + 8 * (size_t)n;
         double2 *ms = W + 9 * (size_t)n, *mp = W + 10 * (size_t)n;
@@ -167,27 +197,8 @@ __device__ bool ac_point(const AcArgs &A, int q, AcTeam<TEAM> &g) {
         // preconditioner coefficients for this frequency, and the start vectors
         double acc0[1] = {0.0};
         for (int i = r0 + threadIdx.x; i < r1; i += blockDim.x) {
-            double2 cs = make_double2(0.0, 0.0), cp = make_double2(0.0, 0.0);
-            const uint32_t ds = A.diag_slot[i];
-            const double2 aii = ds == kSentinel ? make_double2(0.0, 0.0) : cval(A, ds, w);
-            const int pi = A.partner[i];
-            if (A.precond == kPcNone) {
-                cs = make_double2(1.0, 0.0);
-            } else if (A.precond == kPcAuto && pi >= 0) {
-                // [[a_ii a_ik] [a_ki a_kk]]^-1, the row-i half
-                const uint32_t dk = A.diag_slot[pi];
-                const double2 akk = dk == kSentinel ? make_double2(0.0, 0.0) : cval(A, dk, w);
-                const double2 aik = cval(A, A.off_slot[i], w), aki = cval(A, A.off_slot[pi], w);
-                const double2 det = csub(cmul(aii, akk), cmul(aik, aki));
-                if (cabs2(det) > 1e-300) {
-                    cs = cdiv(akk, det);
-                    cp = cdiv(make_double2(-aik.x, -aik.y), det);
-                }
-            } else if (cabs2(aii) > 1e-30) {
-                cs = cdiv(make_double2(1.0, 0.0), aii);        // gpu.rs:300-313
-            } else if (A.precond == kPcAuto) {
-                cs = make_double2(1.0, 0.0);
-            }
+            double2 cp;
+            const double2 cs = ac_precond(A, i, w, cp);
             ms[i] = cs;
             mp[i] = cp;
             const double2 bi = A.b[i];
@@ -372,7 +383,395 @@ __global__ void __launch_bounds__(BLOCK) ac_sweep_kernel(AcArgs A) {
     }
 }
 
+// ---------------------------------------------------------- cluster form --
+// One frequency point per thread-block cluster, everything that an iteration
+// touches on the chip: p, v, r (s), t, r_hat, the preconditioner and the
+// gathered vector z = M^-1 p or M^-1 s of each block's rows in shared memory
+// (112 bytes a row), the matrix in 32-row slices (G and j w C apart, 16-bit
+// local columns) streamed from L2, where all points share it.  Blocks meet at
+// cluster barriers: own z, one barrier, the halo rows of z fetched once each
+// from their owners' shared memory, the product, one reduction.  The
+// recurrence's scalars are updated by one lane inside the reductions.
+//
+// What bounds it: latency (five cluster barriers and reductions an iteration)
+// and issued instructions, so a cluster is the smallest that holds a point
+// (throughput is points in flight / time per iteration, and the fixed part of
+// an iteration does not shrink with more blocks; 10,002 rows x 90 points on
+// clusters of 5 / 6 / 8 / 10 / 16: 71 / 75 / 85 / 92 / 140 ms).  The block and
+// team forms above keep their vectors in global memory (158 MB for those 90
+// points, more than L2 holds).  Before -> after: 10,002 rows x 90 points 160
+// -> 60 ms, 3,002 x 90 33 -> 15 ms, 902 x 90 11.0 -> 4.3 ms, 902 x 540 24 ->
+// 15 ms, 92 x 720 9.9 -> 9.7 ms, 30,602 x 27 361 -> 109 ms, so every system
+// that fits a cluster of 16 takes this form.
+constexpr int kAcClusterBlock = 512;
+constexpr int kAcClusterMax = 16;
+constexpr int kAcRowBytes = 7 * 16;        // p v r t rh ms z
+
+struct AcClusterArgs {
+    int C, smem_bytes, any_pair;
+    const uint32_t *sl_ptr;                // per 32-row slice of each block: first entry / 32 (slice_base[b] + s)
+    const uint32_t *slice_base;            // per block: first slice in sl_ptr
+    const uint16_t *col;                   // local columns, 32 entries per slice column
+    const double *gval, *cval;             // G and C in the same places (cval may be null)
+    const uint32_t *halo_ptr, *halo;       // per block: places of its halo rows
+    const uint32_t *pair_ptr, *pair_row;   // per block: its rows in 2x2 pairs (local index) ...
+    const uint32_t *pair_place;            // ... and their partners' places
+    const uint32_t *place_partner;         // per row in a pair: the partner's place
+};
+
+// A place: block rank in the upper bits, local row in the lower; for a halo
+// row, bit kPlacePaired marks half of a 2x2 pair.
+constexpr uint32_t kPlaceBits = 20, kPlacePaired = 0x80000000u;
+
+struct AcScalars {
+    double2 beta, om, al, omega, rho, rho_new;
+    double rr, rh2, bnorm, abs_tol, tol2, rnorm;
+    int phase, restart, code, it, restarts, q;
+};
+
+// Entry of an own-row array (at the same offset in every block) at a place.
+__device__ __forceinline__ double2 ld_place(const double2 *base, uint32_t place) {
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(base + (place & ((1u << kPlaceBits) - 1u)));
+    uint32_t r;
+    double2 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                 : "=r"(r) : "r"(a), "r"((place & ~kPlacePaired) >> kPlaceBits));
+    asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(r) : "memory");
+    return v;
+}
+
+// !(sqrt(x) >= rel sqrt(y)) through squares (see below_root()).
+__device__ __forceinline__ bool root_below_root(double x, double rel, double y) {
+    const double y2 = rel * rel * y;
+    if (x > 1e-290 && x < 1e290 && y2 > 1e-290 && y2 < 1e290) return x < y2;
+    return !(sqrt(x) >= rel * sqrt(y));
+}
+
+// One lane: what follows a reduction (totals s), the same tests and order as
+// ac_point().
+__device__ __forceinline__ void ac_scalars_step(AcScalars &q, const double (&s)[4], const AcArgs &A) {
+    bool top = false, restart = false;
+    int code = kKrylovRunning, next = kPhaseDone;
+    const double2 one = make_double2(1.0, 0.0);
+    if (q.phase == kPhaseStart) {
+        q.bnorm = q.rnorm = sqrt(s[0]);
+        q.abs_tol = A.tol * q.bnorm;
+        q.tol2 = q.abs_tol * q.abs_tol;
+        q.rr = q.rh2 = s[0];
+        q.rho_new = make_double2(s[0], 0.0);
+        q.rho = q.al = q.omega = one;
+        q.it = q.restarts = 0;
+        if (!(q.bnorm >= 1e-30)) code = isfinite(q.bnorm) ? kKrylovConverged : kKrylovNan;   // b = 0: x = 0
+        else top = true;
+    } else if (q.phase == kPhaseAB) {
+        const double2 rhv = make_double2(s[0], s[1]);
+        if (root_below_root(cabs2(rhv), kBreakdownRel, q.rh2 * s[2])) {
+            if (q.restarts < A.max_restarts && q.rr > 0.0) {
+                ++q.it;
+                restart = top = true;
+            } else {
+                code = kKrylovBreakRv;
+            }
+        } else {
+            q.al = cdiv(q.rho, rhv);
+            next = kPhaseCD;
+        }
+    } else if (q.phase == kPhaseCD) {              // |s|^2, t^H s, |t|^2
+        if (root_below(s[0], q.abs_tol, q.tol2)) {
+            code = kKrylovConverged;
+            q.rnorm = sqrt(s[0]);
+            ++q.it;
+        } else if (!(s[3] > 0.0)) {
+            code = kKrylovBreakTt;
+        } else {
+            q.omega = cdiv(make_double2(s[1], s[2]), make_double2(s[3], 0.0));
+            next = kPhaseE;
+        }
+    } else {
+        q.rho_new = make_double2(s[0], s[1]);
+        q.rr = s[2];
+        ++q.it;
+        if (!isfinite(s[2])) code = kKrylovNan;
+        else if (root_below(s[2], q.abs_tol, q.tol2)) code = kKrylovConverged;
+        else if (!(cabs2(q.omega) > 1e-60)) code = kKrylovBreakOmega;
+        else top = true;
+    }
+    if (top) {
+        const bool stop = q.it >= A.max_it;
+        if (!restart && !stop && root_below_root(cabs2(q.rho_new), kBreakdownRel, q.rh2 * q.rr)) {
+            if (q.restarts < A.max_restarts && q.rr > 0.0) restart = true;
+            else code = kKrylovBreakRho;
+        }
+        if (stop) code = kKrylovMaxIter;
+        if (restart) {
+            ++q.restarts;
+            q.rho = q.al = q.omega = one;
+            q.rho_new = make_double2(q.rr, 0.0);
+            q.rh2 = q.rr;
+        }
+        if (code == kKrylovRunning) {
+            q.beta = cmul(cdiv(q.rho_new, q.rho), cdiv(q.al, q.omega));
+            q.om = q.omega;
+            q.rho = q.rho_new;
+            next = kPhaseAB;
+        }
+    }
+    if (code != kKrylovRunning && q.phase != kPhaseStart && code != kKrylovConverged) q.rnorm = sqrt(q.rr);
+    if (code == kKrylovConverged && q.phase == kPhaseE) q.rnorm = sqrt(q.rr);
+    q.restart = restart ? 1 : 0;
+    q.code = code;
+    q.phase = code == kKrylovRunning ? next : kPhaseDone;
+}
+
+__global__ void __launch_bounds__(kAcClusterBlock, 1) ac_cluster_kernel(const __grid_constant__ AcArgs A,
+                                                                        const __grid_constant__ AcClusterArgs K) {
+    __shared__ AcScalars S;
+    const int C = K.C, rank = (int)(blockIdx.x % (unsigned)C), n = A.n;
+    const int r0 = (int)(((long long)n * rank) / C), r1 = (int)(((long long)n * (rank + 1)) / C), R = r1 - r0;
+    const int stride = (n + C - 1) / C;            // rows of the largest block: uniform offsets
+    const int lane = threadIdx.x & 31;
+    double2 *p = (double2 *)ohm_dsmem, *v = p + stride, *r = v + stride, *t = r + stride, *rh = t + stride,
+            *ms = rh + stride, *z = ms + stride;
+    const int H = (int)(K.halo_ptr[rank + 1] - K.halo_ptr[rank]);
+    uint32_t *halo = (uint32_t *)(z + R + H + 1);
+    for (int h = threadIdx.x; h < H; h += blockDim.x) halo[h] = K.halo[K.halo_ptr[rank] + h];
+    const uint32_t *sl = K.sl_ptr + K.slice_base[rank];
+    const GridSync none{nullptr, nullptr};
+    reduce_buffers_init();
+    if (C > 1) cluster_barrier();
+    auto team_sync = [&]() { if (C > 1) cluster_barrier(); else __syncthreads(); };
+    for (;;) {
+        // next point: the cluster's first block takes it and tells the others
+        if (rank == 0 && threadIdx.x == 0) {
+            const int q = (int)atomicAdd(A.queue, 1u);
+            for (int k = 0; k < C; ++k) {
+                const uint32_t a = (uint32_t)__cvta_generic_to_shared(&S.q);
+                uint32_t b;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(b) : "r"(a), "r"(k));
+                asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(b), "r"(q) : "memory");
+            }
+        }
+        team_sync();
+        const int q = S.q;
+        if (q >= A.n_freq) return;
+        const double w = A.omega[q];
+        double2 *W = A.work + (size_t)q * A.vecs * n;
+        double2 *x = W + r0, *mp = W + n;           // x and, for 2x2 pairs, the partner's coefficient
+        if (threadIdx.x == 0) S.phase = kPhaseStart;
+        __syncthreads();
+        for (;;) {
+            const int phase = S.phase;
+            if (phase == kPhaseDone) break;
+            double acc[4] = {0.0, 0.0, 0.0, 0.0};
+            if (phase == kPhaseE) {
+                const double2 omega = S.omega;
+#pragma unroll 4
+                for (int li = threadIdx.x; li < R; li += blockDim.x) {
+                    x[li] = cadd(x[li], cmul(omega, z[li]));
+                    const double2 ri = csub(r[li], cmul(omega, t[li]));
+                    r[li] = ri;
+                    const double2 d = cdotc(rh[li], ri);
+                    acc[0] += d.x;
+                    acc[1] += d.y;
+                    acc[2] += cabs2(ri);
+                }
+            } else if (phase != kPhaseStart) {
+                const bool cd = phase == kPhaseCD;
+                const double2 al = S.al;
+                if (!cd && S.restart) {
+#pragma unroll 1
+                    for (int li = threadIdx.x; li < R; li += blockDim.x) {
+                        rh[li] = r[li];
+                        p[li] = make_double2(0.0, 0.0);
+                        v[li] = make_double2(0.0, 0.0);
+                    }
+                }
+                // p's update, or s (kept in r) and x += alpha M^-1 p; z = M^-1 of it
+                const double2 beta = S.beta, om = S.om;
+#pragma unroll 4
+                for (int li = threadIdx.x; li < R; li += blockDim.x) {
+                    double2 u;
+                    if (cd) {
+                        u = csub(r[li], cmul(al, v[li]));
+                        x[li] = cadd(x[li], cmul(al, z[li]));
+                        r[li] = u;
+                    } else {
+                        u = cadd(cmul(csub(p[li], cmul(om, v[li])), beta), r[li]);
+                        p[li] = u;
+                    }
+                    z[li] = cmul(ms[li], u);
+                }
+                team_sync();
+                double2 *u = cd ? r : p;
+#pragma unroll 2
+                for (int h = threadIdx.x; h < H; h += blockDim.x) {
+                    const uint32_t at = halo[h];
+                    if (!(at & kPlacePaired)) {
+                        z[R + h] = ld_place(z, at);
+                    } else {
+                        const int q1 = (int)((at & ~kPlacePaired) >> kPlaceBits);
+                        const int j = (int)(((long long)n * q1) / C) + (int)(at & ((1u << kPlaceBits) - 1u));
+                        z[R + h] = cadd(cmul(ld_place(ms, at), ld_place(u, at)), cmul(mp[j], ld_place(u, K.place_partner[j])));
+                    }
+                }
+                if (K.any_pair) {
+                    const uint32_t k1 = K.pair_ptr[rank + 1];
+                    for (uint32_t k = K.pair_ptr[rank] + threadIdx.x; k < k1; k += blockDim.x) {
+                        const int li = (int)K.pair_row[k];
+                        z[li] = cadd(z[li], cmul(mp[r0 + li], ld_place(u, K.pair_place[k])));
+                    }
+                }
+                __syncthreads();
+#pragma unroll 1
+                for (int li = threadIdx.x; li - lane < R; li += blockDim.x) {
+                    const uint32_t e = sl[(li >> 5) + 1] * 32u;
+                    uint32_t k = sl[li >> 5] * 32u + lane;
+                    double2 y = make_double2(0.0, 0.0);
+#pragma unroll 5
+                    for (; k < e; k += 32u) {
+                        const double2 a = make_double2(K.gval[k], K.cval ? w * K.cval[k] : 0.0);
+                        y = cadd(y, cmul(a, z[K.col[k]]));
+                    }
+                    if (li < R) {
+                        if (cd) {
+                            const double2 si = r[li], d = cdotc(y, si);
+                            t[li] = y;
+                            acc[0] += cabs2(si);
+                            acc[1] += d.x;
+                            acc[2] += d.y;
+                            acc[3] += cabs2(y);
+                        } else {
+                            const double2 d = cdotc(rh[li], y);
+                            v[li] = y;
+                            acc[0] += d.x;
+                            acc[1] += d.y;
+                            acc[2] += cabs2(y);
+                        }
+                    }
+                }
+            } else {
+#pragma unroll 1
+                for (int li = threadIdx.x; li < R; li += blockDim.x) {
+                    const int i = r0 + li;
+                    double2 cp;
+                    ms[li] = ac_precond(A, i, w, cp);
+                    if (K.any_pair) mp[i] = cp;
+                    const double2 bi = A.b[i];
+                    x[li] = make_double2(0.0, 0.0);
+                    r[li] = bi;
+                    rh[li] = bi;
+                    p[li] = make_double2(0.0, 0.0);
+                    v[li] = make_double2(0.0, 0.0);
+                    acc[0] += cabs2(bi);
+                }
+                if (threadIdx.x == 0) z[R + H] = make_double2(0.0, 0.0);   // the padding's column
+            }
+            // never false: no counter barrier in a cluster
+            team_reduce_then<4, false>(C, rank, C > 1, nullptr, none, acc, [&](const double (&s)[4], bool writer) {
+                if (writer) ac_scalars_step(S, s, A);
+            });
+        }
+        if (rank == 0 && threadIdx.x == 0) {
+            AcDev &d = A.info[q];
+            d.code = S.code;
+            d.iterations = S.it;
+            d.restarts = S.restarts;
+            d.rnorm = S.rnorm;
+            d.bnorm = S.bnorm;
+        }
+        team_sync();                                // S and the vectors are reused
+    }
+}
+
 using AcFn = void (*)(AcArgs);
+
+// Host side of the cluster form: per block of a cluster of C, the halo rows
+// and the 32-row matrix slices with local columns (entries filled from the G
+// and C values).
+struct AcSlices {
+    int C = 0, smem_bytes = 0;
+    std::vector<uint32_t> sl_ptr, slice_base, halo_ptr, halo, pair_ptr, pair_row, pair_place, place_partner;
+    std::vector<uint16_t> col;
+    std::vector<double> g, c;
+
+    // The smallest cluster whose blocks hold their part of a point in `avail`
+    // bytes of shared memory; false when none does.
+    bool build(int64_t n, const uint32_t *rp, const uint32_t *cl, const double *gv, const double *cv, int64_t avail,
+               const std::vector<int32_t> &partner) {
+        bool ok = false;
+        for (C = 1; C <= kAcClusterMax && !ok; ++C)
+            ok = ((n + C - 1) / C) * kAcRowBytes + 16 * 64 <= avail && fill(n, rp, cl, gv, cv, avail);
+        if (!ok) return false;
+        --C;
+        // halo rows and partners as places
+        auto place = [&](int64_t j) -> uint32_t {
+            int64_t q = (j * C) / n;
+            while (j >= n * (q + 1) / C) ++q;
+            return (uint32_t)((q << kPlaceBits) | (j - n * q / C));
+        };
+        for (uint32_t &h : halo) h = place(h) | (partner[h] >= 0 ? kPlacePaired : 0u);
+        pair_ptr.assign(1, 0);
+        place_partner.assign(n, 0);
+        for (int b = 0; b < C; ++b) {
+            const int64_t r0 = n * b / C, r1 = n * (b + 1) / C;
+            for (int64_t i = r0; i < r1; ++i) {
+                if (partner[i] < 0) continue;
+                place_partner[i] = place(partner[i]);
+                pair_row.push_back((uint32_t)(i - r0));
+                pair_place.push_back(place_partner[i]);
+            }
+            pair_ptr.push_back((uint32_t)pair_row.size());
+        }
+        return true;
+    }
+    bool fill(int64_t n, const uint32_t *rp, const uint32_t *cl, const double *gv, const double *cv, int64_t avail) {
+        const int64_t stride = (n + C - 1) / C, nnz = rp[n];
+        std::vector<int32_t> at(n, -1);
+        sl_ptr.clear(); slice_base.clear(); halo.clear(); col.clear(); g.clear(); c.clear();
+        halo_ptr.assign(1, 0);
+        uint32_t w_total = 0;
+        size_t h_max = 0;
+        for (int b = 0; b < C; ++b) {
+            const int64_t r0 = n * b / C, r1 = n * (b + 1) / C, R = r1 - r0;
+            const size_t h0 = halo.size();
+            for (uint32_t k = rp[r0]; k < rp[r1]; ++k) {
+                const int64_t j = cl[k];
+                if ((j >= r0 && j < r1) || at[j] >= 0) continue;
+                at[j] = (int32_t)(R + (int64_t)(halo.size() - h0));
+                halo.push_back((uint32_t)j);
+            }
+            const size_t H = halo.size() - h0;
+            h_max = std::max(h_max, H);
+            if (R + (int64_t)H >= 0xFFFF) return false;
+            slice_base.push_back((uint32_t)sl_ptr.size());
+            for (int64_t s = r0; s < r1; s += 32) {
+                uint32_t width = 0;
+                for (int64_t i = s; i < std::min(r1, s + 32); ++i) width = std::max(width, rp[i + 1] - rp[i]);
+                sl_ptr.push_back(w_total);
+                w_total += width;
+                if (32ull * w_total > 2ull * (uint64_t)nnz + 4096) return false;    // rows too uneven to pad
+                const size_t e0 = g.size();
+                g.resize(e0 + 32ull * width, 0.0);
+                c.resize(e0 + 32ull * width, 0.0);
+                col.resize(e0 + 32ull * width, (uint16_t)(R + (int64_t)H));
+                for (int64_t i = s; i < std::min(r1, s + 32); ++i)
+                    for (uint32_t k = rp[i]; k < rp[i + 1]; ++k) {
+                        const size_t e = e0 + 32ull * (k - rp[i]) + (size_t)(i - s);
+                        const int64_t j = cl[k];
+                        g[e] = gv[k];
+                        c[e] = cv ? cv[k] : 0.0;
+                        col[e] = (uint16_t)(j >= r0 && j < r1 ? j - r0 : at[j]);
+                    }
+            }
+            sl_ptr.push_back(w_total);
+            for (size_t h = h0; h < halo.size(); ++h) at[halo[h]] = -1;
+            halo_ptr.push_back((uint32_t)halo.size());
+        }
+        const int64_t bytes = stride * kAcRowBytes + 16 * ((int64_t)h_max + 1) + 4 * (int64_t)h_max + 16;
+        smem_bytes = (int)bytes;
+        return bytes <= avail;
+    }
+};
 
 AcFn pick_ac(double avg, bool wide) {
     if (wide) {
@@ -414,8 +813,38 @@ extern "C" ohm_status ohm_ac_sweep(ohm_ctx *c, int64_t n, int64_t nnz, const uin
     std::vector<char> touched(nnz, 0);
     PcHost pc;
     build_precond(n, row_ptr, col, g_values, touched, params->precond == OHM_PRECOND_AUTO, pc);
+    // cluster form where a point fits a cluster's shared memory
+    AcSlices slices;
+    AcClusterArgs K{};
+    int clusters = 0;
+    cudaLaunchAttribute cl_attr[1];
+    cudaLaunchConfig_t cl_cfg = {};
+    if (n >= 1) {
+        int optin = 0;
+        cudaFuncAttributes fa{};
+        if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device) == cudaSuccess &&
+            cudaFuncGetAttributes(&fa, ac_cluster_kernel) == cudaSuccess &&
+            slices.build(n, row_ptr, col, g_values, c_values, (int64_t)optin - (int64_t)fa.sharedSizeBytes - 1024,
+                         pc.partner) &&
+            cudaFuncSetAttribute(ac_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 slices.smem_bytes) == cudaSuccess &&
+            cudaFuncSetAttribute(ac_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+            cl_attr[0].id = cudaLaunchAttributeClusterDimension;
+            cl_attr[0].val.clusterDim.x = (unsigned)slices.C;
+            cl_attr[0].val.clusterDim.y = cl_attr[0].val.clusterDim.z = 1;
+            cl_cfg.gridDim = dim3((unsigned)slices.C);
+            cl_cfg.blockDim = dim3(kAcClusterBlock);
+            cl_cfg.dynamicSmemBytes = (size_t)slices.smem_bytes;
+            cl_cfg.stream = c->stream;
+            cl_cfg.attrs = cl_attr;
+            cl_cfg.numAttrs = 1;
+            if (cudaOccupancyMaxActiveClusters(&clusters, ac_cluster_kernel, &cl_cfg) != cudaSuccess) clusters = 0;
+        }
+        (void)cudaGetLastError();
+    }
+    const int vecs = clusters > 0 ? 2 : kAcVecs;
     // frequency groups sized so the per-point workspace stays under ~4 GB
-    const size_t per_point = (size_t)kAcVecs * n * sizeof(double2);
+    const size_t per_point = (size_t)vecs * n * sizeof(double2);
     const int64_t group = std::max<int64_t>(1, std::min<int64_t>(n_freq, ((size_t)4 << 30) / per_point));
     std::vector<void *> allocs;
     auto put = [&](auto **dst, const auto *src, size_t count) -> cudaError_t {
@@ -441,7 +870,7 @@ extern "C" ohm_status ohm_ac_sweep(ohm_ctx *c, int64_t n, int64_t nnz, const uin
     if (e == cudaSuccess) e = put(&d_diag, pc.diag_slot.data(), n);
     if (e == cudaSuccess) e = put(&d_off, pc.off_slot.data(), n);
     if (e == cudaSuccess) e = put(&d_omega, (const double *)nullptr, group);
-    if (e == cudaSuccess) e = put(&d_work, (const double2 *)nullptr, (size_t)group * kAcVecs * n);
+    if (e == cudaSuccess) e = put(&d_work, (const double2 *)nullptr, (size_t)group * vecs * n);
     if (e == cudaSuccess) e = put(&d_info, (const AcDev *)nullptr, group);
     if (e == cudaSuccess) e = put(&d_queue, (const unsigned int *)nullptr, 1);
     A.n = (int)n;
@@ -453,6 +882,26 @@ extern "C" ohm_status ohm_ac_sweep(ohm_ctx *c, int64_t n, int64_t nnz, const uin
     A.rp = d_rp; A.col = d_col; A.g = d_g; A.c = d_c; A.b = d_b; A.omega = d_omega;
     A.partner = d_partner; A.diag_slot = d_diag; A.off_slot = d_off;
     A.work = d_work; A.info = d_info; A.queue = d_queue;
+    A.vecs = vecs;
+    if (clusters > 0) {
+        K.C = slices.C;
+        K.smem_bytes = slices.smem_bytes;
+        K.any_pair = pc.any_pair ? 1 : 0;
+        uint32_t *u = nullptr;
+        uint16_t *h = nullptr;
+        double *d = nullptr;
+        if (e == cudaSuccess) { e = put(&u, slices.sl_ptr.data(), slices.sl_ptr.size()); K.sl_ptr = u; }
+        if (e == cudaSuccess) { e = put(&u, slices.slice_base.data(), slices.slice_base.size()); K.slice_base = u; }
+        if (e == cudaSuccess) { e = put(&u, slices.halo_ptr.data(), slices.halo_ptr.size()); K.halo_ptr = u; }
+        if (e == cudaSuccess) { e = put(&u, slices.halo.data(), slices.halo.size()); K.halo = u; }
+        if (e == cudaSuccess) { e = put(&u, slices.pair_ptr.data(), slices.pair_ptr.size()); K.pair_ptr = u; }
+        if (e == cudaSuccess) { e = put(&u, slices.pair_row.data(), slices.pair_row.size()); K.pair_row = u; }
+        if (e == cudaSuccess) { e = put(&u, slices.pair_place.data(), slices.pair_place.size()); K.pair_place = u; }
+        if (e == cudaSuccess) { e = put(&u, slices.place_partner.data(), slices.place_partner.size()); K.place_partner = u; }
+        if (e == cudaSuccess) { e = put(&h, slices.col.data(), slices.col.size()); K.col = h; }
+        if (e == cudaSuccess) { e = put(&d, slices.g.data(), slices.g.size()); K.gval = d; }
+        if (e == cudaSuccess && c_values) { e = put(&d, slices.c.data(), slices.c.size()); K.cval = d; }
+    }
     // a point per SM at most: give each point a whole SM when the system is large
     const bool wide = n >= 2048 && n_freq <= c->num_sms;
     const int block = wide ? kAcWideBlock : kAcBlock;
@@ -498,7 +947,7 @@ extern "C" ohm_status ohm_ac_sweep(ohm_ctx *c, int64_t n, int64_t nnz, const uin
         // team sizes: the same base size for every point, one more block for
         // the lowest frequencies while blocks are left
         int teamed = 0;
-        if (team_capable && m < total_blocks) {
+        if (clusters == 0 && team_capable && m < total_blocks) {
             const int base = std::min<int>(tmax, (int)(total_blocks / m));
             int spare = base < tmax ? total_blocks - base * (int)m : 0;
             std::vector<int32_t> by_freq((size_t)m);
@@ -519,7 +968,10 @@ extern "C" ohm_status ohm_ac_sweep(ohm_ctx *c, int64_t n, int64_t nnz, const uin
                 }
             if (base > 1 || h_point_team[by_freq[0]] > 1) teamed = (int)h_blk_point.size();
         }
-        if (teamed > 0) {
+        if (clusters > 0) {
+            cl_cfg.gridDim = dim3((unsigned)(slices.C * (int)std::min<int64_t>(clusters, m)));
+            if (e == cudaSuccess) e = cudaLaunchKernelEx(&cl_cfg, ac_cluster_kernel, A, K);
+        } else if (teamed > 0) {
             A.team_mode = 1;
             if (e == cudaSuccess)
                 e = cudaMemcpyAsync(d_blk_point, h_blk_point.data(), teamed * sizeof(int32_t), cudaMemcpyHostToDevice,
@@ -547,7 +999,7 @@ extern "C" ohm_status ohm_ac_sweep(ohm_ctx *c, int64_t n, int64_t nnz, const uin
         }
         // x of every point: the first of its kAcVecs vectors
         for (int64_t k = 0; e == cudaSuccess && k < m; ++k)
-            e = cudaMemcpyAsync(x_re_im + 2 * (size_t)(f0 + k) * n, d_work + (size_t)k * kAcVecs * n,
+            e = cudaMemcpyAsync(x_re_im + 2 * (size_t)(f0 + k) * n, d_work + (size_t)k * vecs * n,
                                 n * sizeof(double2), cudaMemcpyDeviceToHost, c->stream);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(hinfo.data(), d_info, m * sizeof(AcDev), cudaMemcpyDeviceToHost, c->stream);
