@@ -189,20 +189,26 @@ static int krylov_smem_bytes(const void *fn, int64_t n, int64_t nnz_short, int g
 }
 
 // Grid, shared memory and synchronisation of a grid-team kernel over a
-// system of a.n rows: one block per 1024 rows or devices, at
-// most what is co-resident; up to 16 blocks form one cluster (its barrier
-// takes 0.33 us against 1.0-1.13 us for the counter barrier; measured for 2
-// to 16 blocks, 16 is the largest cluster).
+// system of a.n rows, by the larger of its rows and devices:
+//   up to 1,024: one block, which needs no team barrier (401- and 578-row
+//     systems on two blocks: +22 %);
+//   then one block per 512, as one cluster of up to 16 blocks (its barrier
+//     takes 0.33 us against 1.0-1.13 us for the counter barrier) while a
+//     block's share stays below 1,700, about what its shared memory holds: per
+//     BiCGSTAB iteration 1,602 rows 10.4 -> 9.3 us, 3,602 rows 10.2 -> 9.1
+//     against one block per 1,024; 22,502 rows on 16 blocks 11.4 us, on a grid
+//     of 22 13.6 us;
+//   beyond: one block per 512, at most one per SM (27,227 rows 13.3 -> 12.2
+//     us).
 ohm_status ohm_team_shape(const void *fn, int num_sms, int max_grid, bool slices, int64_t nnz, KernelArgs &a,
                           int &grid) {
     int per_sm = 0;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kBlock, 0));
     if (per_sm < 1) return fail(OHM_ERR_CUDA, "solver kernel does not fit on an SM");
-    per_sm = 1;
-    int64_t want = (a.n + kTeamRows - 1) / kTeamRows;
-    const int64_t ndev = (int64_t)a.nd + a.nq + a.nm;
-    want = std::max<int64_t>(want, (ndev + kTeamRows - 1) / kTeamRows);
-    int64_t cap = (int64_t)per_sm * num_sms;
+    const int64_t items = std::max<int64_t>(a.n, (int64_t)a.nd + a.nq + a.nm);
+    int64_t want = items <= kTeamOneBlock ? 1 : (items + kTeamRows - 1) / kTeamRows;
+    if (items <= kMaxTeamCluster * kTeamClusterRows) want = std::min<int64_t>(want, kMaxTeamCluster);
+    int64_t cap = num_sms;
     if (max_grid > 0) cap = std::min<int64_t>(cap, max_grid);
     grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, cap));
     a.smem_bytes = slices && a.slice_export ? krylov_smem_bytes(fn, a.n, nnz - a.nnz_long, grid) : 0;

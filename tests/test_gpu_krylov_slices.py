@@ -1,8 +1,8 @@
 """Slice layouts of the single-system Krylov solve (csrc/solver_kernel.cuh,
 ``krylov_slice``) against the global-memory solve, which runs the same
 iteration in the same order: the results must be equal bit for bit.  Sizes at
-the edges: one block (up to 1,024 rows), clusters of 2 to 16 blocks, grids
-beyond, ragged 32-row slices, rows of uneven length, pairs whose two rows
+the edges: one block (up to 1,024 rows), clusters of 2 to 16 blocks (up to
+27,200), grids beyond, ragged 32-row slices, rows of uneven length, pairs whose two rows
 belong to different blocks, slices too large for shared memory, several lanes
 per row.  Small systems are also compared with a dense solve.
 """
@@ -49,7 +49,7 @@ def _random_system(n, per_row, seed, wide_rows=0):
     return mna.Csr(n, n, rp, cols, val), rng.standard_normal(n)
 
 
-@pytest.mark.parametrize("n", [1, 31, 33, 1023, 1025, 2049, 16383, 16385, 40007])
+@pytest.mark.parametrize("n", [1, 31, 33, 1024, 1025, 2049, 16385, 27200, 27201, 40007])
 @pytest.mark.parametrize("prec", [0, 1], ids=["fp64", "mixed"])
 def test_sizes(n, prec):
     a, b = _random_system(n, 2, n, wide_rows=n // 500)
@@ -85,6 +85,6 @@ def test_pairs_across_blocks(nodes):
 
 
 def test_slices_larger_than_shared_memory():
-    """2,100 rows a block: the matrix slices stream from global memory."""
+    """2,100 rows a block on 148 SMs: the matrix slices stream from global memory."""
     s = mna.compile_circuit(ck.resistor_ladder(310_000, seed=3))
     _both(s.g, s.b_dc, S.BiCgStabParams(tolerance=1e-12, max_iterations=2000))
