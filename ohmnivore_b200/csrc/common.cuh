@@ -136,6 +136,7 @@ __device__ __forceinline__ void block_max(double (&v)[NV], double *smem) { block
 // cluster): 0.33 us for 2 to 16 blocks of 1024 threads, against 1.0-1.13 us
 // for the counter barrier above.
 __device__ __forceinline__ void cluster_barrier() {
+    __syncwarp();       // the aligned forms want the whole warp together
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 

@@ -485,9 +485,9 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *s
 // inner_rtol * ||r0||).  On success the correction is left in a.dx (FP64)
 // for the rows of this block.
 //
-// This is the global-memory form (batches, systems whose slices do not fit
-// in shared memory); krylov_smem() is the same iteration with each block's
-// slice in shared memory.
+// This is the global-memory form (slices whose gathered vector does not fit in
+// shared memory, and OHM_KRYLOV_LAYOUT_GLOBAL); krylov_slice() is the same
+// iteration with each block's slice in shared memory.
 //
 // Newton solves measure that stopping norm on the diagonally scaled residual
 // W r, w_i = 1/|J_ii| (1 for a zero diagonal): volts instead of amperes, so a
