@@ -471,6 +471,21 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *s
     return before;
 }
 
+// |x| < rel sqrt(y), compared as squares: a square root is 120 cycles on the
+// one lane that every thread waits for.  Where a square would leave the
+// normal range the root decides.  krylov() and krylov_slice() share these
+// tests: blocks of one team may run either form, and all of them have to take
+// the same branch.
+__device__ __forceinline__ bool below_root(double x, double rel, double y) {
+    const double x2 = x * x, y2 = rel * rel * y;
+    if (x2 > 1e-290 && x2 < 1e290 && y2 > 1e-290 && y2 < 1e290) return x2 < y2;
+    return !(fabs(x) >= rel * sqrt(y));
+}
+// sqrt(y) < tol, tol2 = tol^2.
+__device__ __forceinline__ bool root_below(double y, double tol, double tol2) {
+    return tol2 > 1e-290 && tol2 < 1e290 ? y < tol2 : sqrt(y) < tol;
+}
+
 // Right-preconditioned BiCGSTAB on J d = r64 in precision T, d0 = 0, with
 // the reference's operation order (bicgstab.rs:104-183) and three grid
 // synchronisations per iteration:
@@ -553,7 +568,7 @@ __device__ __forceinline__ int krylov(const KernelArgs &a, Team &g, double tol_f
         if (!g.template allreduce<2>(acc0)) return kKrylovAbort;
     }
     const double r0norm = sqrt(acc0[1]);            // stopping norm (scaled for Newton)
-    const double abs_tol = fmax(tol_floor, inner_rtol * r0norm);
+    const double abs_tol = fmax(tol_floor, inner_rtol * r0norm), tol2 = abs_tol * abs_tol;
     double rr_cur = acc0[0];          // ||r||^2
     double rhat2 = acc0[0];           // ||r_hat||^2
     double rho_new = acc0[0];         // (r_hat, r)
@@ -593,7 +608,7 @@ __device__ __forceinline__ int krylov(const KernelArgs &a, Team &g, double tol_f
         code = kKrylovConverged;
     } else {
         for (; it < max_it; ++it) {
-            if (!(fabs(rho_new) >= kBreakdownRel * sqrt(rhat2 * rr_cur))) {
+            if (below_root(rho_new, kBreakdownRel, rhat2 * rr_cur)) {
                 if (out.restarts < a.max_restarts && rr_cur > 0.0) {
                     OHM_RESTART();
                 } else {
@@ -634,8 +649,16 @@ __device__ __forceinline__ int krylov(const KernelArgs &a, Team &g, double tol_f
             {
                 if (!g.template allreduce<2>(acc1)) return kKrylovAbort;
             }
-            if (!(fabs(acc1[0]) >= kBreakdownRel * sqrt(rhat2 * acc1[1]))) {
+            if (below_root(acc1[0], kBreakdownRel, rhat2 * acc1[1])) {
                 if (out.restarts < a.max_restarts && rr_cur > 0.0) {
+                    if (it + 1 >= max_it) {
+                        // the limit comes first, with no restart and no sync,
+                        // as in krylov_scalars_step()
+                        ++out.restarts;
+                        ++it;
+                        code = kKrylovMaxIter;
+                        break;
+                    }
                     OHM_RESTART();        // cur still holds r; restart from it
                     continue;
                 }
@@ -679,7 +702,7 @@ __device__ __forceinline__ int krylov(const KernelArgs &a, Team &g, double tol_f
             {
                 if (!g.template allreduce<4>(acc3)) return kKrylovAbort;
             }
-            if (sqrt(acc3[3]) < abs_tol) {          // early exit (bicgstab.rs:134-139)
+            if (root_below(acc3[3], abs_tol, tol2)) {   // early exit (bicgstab.rs:134-139)
                 for (int i = r0 + threadIdx.x; i < r1; i += blockDim.x) {
                     const T ph = phat_own(i, own(nxt, i));
                     d[i - r0] = cvt<T>((double)d[i - r0] + al * (double)ph);
@@ -715,11 +738,10 @@ __device__ __forceinline__ int krylov(const KernelArgs &a, Team &g, double tol_f
             { KRec<T> *tmp = cur; cur = nxt; nxt = tmp; }
             rho_new = acc4[0];
             rr_cur = acc4[1];
-            const double rnorm = sqrt(acc4[2]);
-            if (!isfinite(rnorm)) { code = kKrylovNan; ++it; break; }
-            if (rnorm < abs_tol) { code = kKrylovConverged; ++it; break; }
+            if (!isfinite(acc4[2])) { code = kKrylovNan; ++it; break; }
+            if (root_below(acc4[2], abs_tol, tol2)) { code = kKrylovConverged; ++it; break; }
             if (fabs(omega) < 1e-30) { code = kKrylovBreakOmega; ++it; break; }
-            if (accept_partial && it + 1 == max_it && rnorm <= 0.5 * r0norm) {
+            if (accept_partial && it + 1 == max_it && sqrt(acc4[2]) <= 0.5 * r0norm) {
                 code = kKrylovConverged;          // inexact inner solve accepted
                 ++it;
                 break;
@@ -980,19 +1002,6 @@ struct KrylovScalars {
     double rho, rho_new, rr, rhat2, abs_tol, r0norm, tol2;
     int phase, restart, early, code, it, restarts, flip;
 };
-
-// |x| < rel sqrt(y), compared as squares: a square root is 120 cycles on the
-// one lane that every thread waits for.  Where a square would leave the
-// normal range the root decides.
-__device__ __forceinline__ bool below_root(double x, double rel, double y) {
-    const double x2 = x * x, y2 = rel * rel * y;
-    if (x2 > 1e-290 && x2 < 1e290 && y2 > 1e-290 && y2 < 1e290) return x2 < y2;
-    return !(fabs(x) >= rel * sqrt(y));
-}
-// sqrt(y) < tol, tol2 = tol^2.
-__device__ __forceinline__ bool root_below(double y, double tol, double tol2) {
-    return tol2 > 1e-290 && tol2 < 1e290 ? y < tol2 : sqrt(y) < tol;
-}
 
 // What follows a reduction: s holds its totals, q the scalars.
 struct KrylovLimits {

@@ -1,0 +1,128 @@
+"""Teams whose blocks run different forms of the Krylov solve
+(csrc/solver_kernel.cuh): a block whose slice does not fit in shared memory
+runs krylov() beside blocks that run krylov_slice().  Both have to meet at the
+same barriers, take the same branches and give the global-memory layout's bits.
+
+``_layouts`` restates the rule by which each block chooses, so that a test can
+tell that the layout it is about is the one that ran.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+import torch  # noqa: E402
+
+from ohmnivore_b200 import _lib, mna  # noqa: E402
+from ohmnivore_b200 import solver as S  # noqa: E402
+
+BLOCK_BYTES = 227 * 1024          # shared memory of one block
+STATIC_BYTES = 4096               # at least the kernels' static part and the reserve
+
+
+def _blocks(n):
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    if n <= 1024:
+        return 1
+    want = -(-n // 512)
+    return min(want, 16) if n <= 27200 else min(want, sms)
+
+
+def _up16(b):
+    return (b + 15) // 16 * 16
+
+
+def _layouts(a, room=BLOCK_BYTES - STATIC_BYTES):
+    """Per block of a system with one lane per row and no long rows: "chip",
+    "stream" or "none" (slice_map(), slice_offsets())."""
+    n, blocks, rp, col = a.nrows, _blocks(a.nrows), np.asarray(a.row_ptr), np.asarray(a.col)
+    assert len(col) <= 5.5 * n
+    rows = -(-n // blocks) + 1
+    nnz_blk = int(len(col) * rows / n * 1.15) + 512
+    halo = min(nnz_blk, 4096) if blocks > 1 else 0
+    room = min(rows * 9 + rows // 8 + halo * 12 + 256 + rows * 64 + nnz_blk * 10, room) // 16 * 16
+    bits = 0
+    while 8 << (bits + 1) <= room // 2 and bits < 14:
+        bits += 1
+    table = 1 << bits if blocks > 1 else 0
+    out = []
+    for b in range(blocks):
+        r0, r1 = n * b // blocks, n * (b + 1) // blocks
+        r = r1 - r0
+        near = col[rp[r0]:rp[r1]]
+        h = len(np.unique(near[(near < r0) | (near >= r1)]))
+        width = np.diff(rp[r0:r1 + 1])
+        w = int(sum(width[s:s + 32].max() for s in range(0, r, 32)))
+
+        def offsets(w):
+            z = _up16(4 * ((r + 31) // 32 + 1)) + _up16(4 * h) + _up16(r) + 64 * w
+            vec = z + _up16(8 * (r + h + 1))
+            return z, vec, vec + 8 * _up16(8 * r) + 256 * w
+
+        z, _, end = offsets(w)
+        z0, vec0, _ = offsets(0)
+        if h >= table // 4 * 3 and blocks > 1 or r + h >= 0xFFFF or w > 0xFFFF:
+            out.append("none")
+        elif end <= room and z <= room - 8 * table:
+            out.append("chip")
+        elif vec0 > room or z0 > room - 8 * table:
+            out.append("none")
+        else:
+            start = lambda k: k + k // 4  # noqa: E731
+            out.append("stream" if 32 * w <= start(int(rp[r1])) - start(int(rp[r0])) else "none")
+    return out
+
+
+def _solve(a, b, params):
+    """(x or None, info) in the automatic and in the global-memory layout."""
+    ctx = S.Context(0)
+    out = []
+    try:
+        for layout in (_lib.KRYLOV_LAYOUT_AUTO, _lib.KRYLOV_LAYOUT_GLOBAL):
+            ctx.set_krylov_layout(layout)
+            solver = S.GpuSolver(ctx, params)
+            x = None
+            try:
+                x = solver.solve_real(a, b)
+            except S.SolveError:
+                pass
+            out.append((x, solver.last_info))
+    finally:
+        ctx.close()
+    return out
+
+
+def _csr(n, rows, cols, vals):
+    order = np.lexsort((cols, rows))
+    rp = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=n))])
+    return mna.Csr(n, n, rp, cols[order], vals[order])
+
+
+def _skew(n, wide):
+    """2x2 skew blocks [[0 1] [-1 0]]; row 0 also has `wide` entries +1, -1,
+    +1, ...: (b, A b) = 0 exactly for b = 1, and row 0's block keeps no slice."""
+    k = np.arange(n)
+    far = 2 + np.arange(wide)
+    rows = np.concatenate([k, np.zeros(wide, np.int64)])
+    cols = np.concatenate([k ^ 1, far])
+    vals = np.concatenate([np.where(k % 2 == 0, 1.0, -1.0), np.where(far % 2 == 0, 1.0, -1.0)])
+    return _csr(n, rows, cols, vals)
+
+
+@pytest.mark.parametrize("max_it,restarts,code", [(1, 1, 2), (3, 3, 2), (100, 50, 4)])
+@pytest.mark.parametrize("prec", [0, 1], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("n", [4000, 30000])
+def test_breakdown_at_the_iteration_limit(n, prec, max_it, restarts, code):
+    """(r_hat, v) = 0 in every iteration: each one restarts, the last one
+    allowed ends the solve (code 2), or the 51st breakdown does (code 4).  A
+    block that met one barrier more or less than the others would make the call
+    time out, or the FP64 solve after the failed FP32 one read partial sums that
+    nobody wrote."""
+    a = _skew(n, 2000)
+    kinds = _layouts(a)
+    assert kinds[0] == "none" and set(kinds[1:]) == {"chip"}
+    params = S.BiCgStabParams(tolerance=1e-10, max_iterations=max_it, precond=_lib.PRECOND_NONE, precision=prec)
+    for x, info in _solve(a, np.ones(n), params):
+        assert x is None and info["status"] == _lib.ERR_SOLVE and info["krylov_code"] == code
+        assert info["krylov_restarts"] == (1 + prec) * restarts
+        assert info["fp64_fallbacks"] == prec
