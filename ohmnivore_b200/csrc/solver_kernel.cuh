@@ -471,6 +471,16 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *s
     return before;
 }
 
+// A breakdown at a residual more than ten times the initial one (||W r||,
+// compared as squares) gives the solve's work up, once: back to d = 0 and
+// r = r64, with the shadow residual r64 + g r, g = ||r64|| / ||r|| (its product
+// with r64 is not small: a breakdown of rho makes r orthogonal to the first
+// shadow residual).  Such breakdowns come after a spike of the recurrence; 4
+// of 440 solves of a 600 x 600 diode mesh (1.0 V, 5 % diodes) met one, at 140 to
+// 2.6e8 times the initial residual, and one of them then spent the rest of its
+// 20,000 iterations above it.
+constexpr double kRestartFromStart = 100.0;
+
 // |x| < rel sqrt(y), compared as squares: a square root is 120 cycles on the
 // one lane that every thread waits for.  Where a square would leave the
 // normal range the root decides.  krylov() and krylov_slice() share these
@@ -529,50 +539,12 @@ __device__ __forceinline__ int krylov(const KernelArgs &a, Team &g, double tol_f
     auto own = [&](KRec<T> *buf, int i) -> KRec<T> { return buf[i]; };
     auto is_paired = [&](int i) -> bool { return partner[i] >= 0; };
 
-    // ---- start: r = r64, r_hat = r, p = v = d = 0; preconditioner coefficients ----
-    double acc0[2] = {0.0, 0.0};     // ||r||^2, ||W r||^2
-    for (int i = r0 + threadIdx.x; i < r1; i += blockDim.x) {
-        const int li = i - r0;
-        const T rt = cvt<T>(a.r64[i]);
-        double cs = 0.0, cp = 0.0;
-        const uint32_t ds = a.diag_slot[i];
-        const double aii = ds == kSentinel ? 0.0 : a.vals64[ds];
-        const double wi = (wt && fabs(aii) > 1e-30) ? 1.0 / fabs(aii) : 1.0;
-        if (wt) w[li] = wi;
-        if (a.precond != kPcNone) {
-            const int pi = partner[i];
-            if (a.precond == kPcAuto && pi >= 0) {
-                const double akk = a.diag_slot[pi] == kSentinel ? 0.0 : a.vals64[a.diag_slot[pi]];
-                const double aik = a.vals64[a.off_slot[i]];
-                const double aki = a.vals64[a.off_slot[pi]];
-                const double det = aii * akk - aik * aki;
-                if (fabs(det) > 1e-300) { cs = akk / det; cp = -aik / det; }
-            } else if (fabs(aii) > 1e-30) {
-                cs = 1.0 / aii;
-            } else if (a.precond == kPcAuto) {
-                cs = 1.0;   // unpaired zero diagonal: identity keeps M^-1 nonsingular
-            }
-        } else {
-            cs = 1.0;
-        }
-        KRec<T> q;
-        q.p = T(0); q.v = T(0); q.r = rt; q.c = cvt<T>(cs);
-        cur[i] = q;
-        pc_part[i] = cvt<T>(cp);
-        rhat[li] = rt;
-        d[li] = T(0);
-        acc0[0] += (double)rt * (double)rt;
-        acc0[1] += (wi * (double)rt) * (wi * (double)rt);
-    }
-    {
-        if (!g.template allreduce<2>(acc0)) return kKrylovAbort;
-    }
-    const double r0norm = sqrt(acc0[1]);            // stopping norm (scaled for Newton)
-    const double abs_tol = fmax(tol_floor, inner_rtol * r0norm), tol2 = abs_tol * abs_tol;
-    double rr_cur = acc0[0];          // ||r||^2
-    double rhat2 = acc0[0];           // ||r_hat||^2
-    double rho_new = acc0[0];         // (r_hat, r)
-    double rho = 1.0, alpha = 1.0, omega = 1.0;
+    double r0norm = 0.0, abs_tol = 0.0, tol2 = 0.0;     // stopping norm (scaled for Newton)
+    double rr0 = 0.0, rw0 = 0.0;
+    double rr_cur = 0.0, rw_cur = 0.0;    // ||r||^2, ||W r||^2
+    double rhat2 = 0.0;                   // ||r_hat||^2
+    double rho_new = 0.0;                 // (r_hat, r)
+    double rho = 1.0, alpha = 1.0, omega = 1.0, mix = 0.0;
     int code = kKrylovRunning;
     int it = 0;
 
@@ -602,14 +574,69 @@ __device__ __forceinline__ int krylov(const KernelArgs &a, Team &g, double tol_f
         return cvt<T>(z);
     };
 
-    if (!isfinite(r0norm)) {
-        code = kKrylovNan;
-    } else if (r0norm < abs_tol || r0norm == 0.0) {
-        code = kKrylovConverged;
-    } else {
+    for (bool again = false;; again = true) {       // twice at most (kRestartFromStart)
+        // ---- start: r = r64, r_hat = r (again: r64 + g r), p = v = d = 0;
+        //      preconditioner coefficients ----
+        double acc0[4] = {0.0, 0.0, 0.0, 0.0};     // ||r||^2, ||W r||^2, (r_hat, r), ||r_hat||^2
+        KRec<T> *const old = cur;
+        cur = (KRec<T> *)a.rec0;
+        nxt = (KRec<T> *)a.rec1;
+        for (int i = r0 + threadIdx.x; i < r1; i += blockDim.x) {
+            const int li = i - r0;
+            const T rt = cvt<T>(a.r64[i]);
+            double cs = 0.0, cp = 0.0;
+            const uint32_t ds = a.diag_slot[i];
+            const double aii = ds == kSentinel ? 0.0 : a.vals64[ds];
+            const double wi = (wt && fabs(aii) > 1e-30) ? 1.0 / fabs(aii) : 1.0;
+            if (wt) w[li] = wi;
+            if (a.precond != kPcNone) {
+                const int pi = partner[i];
+                if (a.precond == kPcAuto && pi >= 0) {
+                    const double akk = a.diag_slot[pi] == kSentinel ? 0.0 : a.vals64[a.diag_slot[pi]];
+                    const double aik = a.vals64[a.off_slot[i]];
+                    const double aki = a.vals64[a.off_slot[pi]];
+                    const double det = aii * akk - aik * aki;
+                    if (fabs(det) > 1e-300) { cs = akk / det; cp = -aik / det; }
+                } else if (fabs(aii) > 1e-30) {
+                    cs = 1.0 / aii;
+                } else if (a.precond == kPcAuto) {
+                    cs = 1.0;   // unpaired zero diagonal: identity keeps M^-1 nonsingular
+                }
+            } else {
+                cs = 1.0;
+            }
+            const T rh = again ? cvt<T>(fma(mix, (double)old[i].r, (double)rt)) : rt;
+            KRec<T> q;
+            q.p = T(0); q.v = T(0); q.r = rt; q.c = cvt<T>(cs);
+            cur[i] = q;
+            pc_part[i] = cvt<T>(cp);
+            rhat[li] = rh;
+            d[li] = T(0);
+            acc0[0] += (double)rt * (double)rt;
+            acc0[1] += (wi * (double)rt) * (wi * (double)rt);
+            acc0[2] += (double)rh * (double)rt;
+            acc0[3] += (double)rh * (double)rh;
+        }
+        {
+            if (!g.template allreduce<4>(acc0)) return kKrylovAbort;
+        }
+        rr_cur = acc0[0]; rw_cur = acc0[1]; rho_new = acc0[2]; rhat2 = acc0[3];
+        rho = 1.0; alpha = 1.0; omega = 1.0;
+        if (!again) {
+            rr0 = rr_cur;
+            rw0 = rw_cur;
+            r0norm = sqrt(rw_cur);
+            abs_tol = fmax(tol_floor, inner_rtol * r0norm);
+            tol2 = abs_tol * abs_tol;
+            if (!isfinite(r0norm)) { code = kKrylovNan; break; }
+            if (r0norm < abs_tol || r0norm == 0.0) { code = kKrylovConverged; break; }
+        }
+        bool back = false;
         for (; it < max_it; ++it) {
             if (below_root(rho_new, kBreakdownRel, rhat2 * rr_cur)) {
                 if (out.restarts < a.max_restarts && rr_cur > 0.0) {
+                    back = !again && rw_cur > kRestartFromStart * rw0;
+                    if (back) break;
                     OHM_RESTART();
                 } else {
                     code = kKrylovBreakRho;
@@ -659,6 +686,8 @@ __device__ __forceinline__ int krylov(const KernelArgs &a, Team &g, double tol_f
                         code = kKrylovMaxIter;
                         break;
                     }
+                    back = !again && rw_cur > kRestartFromStart * rw0;
+                    if (back) { ++it; break; }
                     OHM_RESTART();        // cur still holds r; restart from it
                     continue;
                 }
@@ -738,6 +767,7 @@ __device__ __forceinline__ int krylov(const KernelArgs &a, Team &g, double tol_f
             { KRec<T> *tmp = cur; cur = nxt; nxt = tmp; }
             rho_new = acc4[0];
             rr_cur = acc4[1];
+            rw_cur = acc4[2];
             if (!isfinite(acc4[2])) { code = kKrylovNan; ++it; break; }
             if (root_below(acc4[2], abs_tol, tol2)) { code = kKrylovConverged; ++it; break; }
             if (fabs(omega) < 1e-30) { code = kKrylovBreakOmega; ++it; break; }
@@ -747,7 +777,12 @@ __device__ __forceinline__ int krylov(const KernelArgs &a, Team &g, double tol_f
                 break;
             }
         }
-        if (code == kKrylovRunning) code = kKrylovMaxIter;
+        if (!back) {
+            if (code == kKrylovRunning) code = kKrylovMaxIter;
+            break;
+        }
+        mix = sqrt(rr0 / rr_cur);
+        ++out.restarts;
     }
 #undef OHM_RESTART
     out.iterations = it;
@@ -1000,7 +1035,8 @@ enum KrylovPhase : int { kPhaseStart, kPhaseAB, kPhaseCD, kPhaseE, kPhaseDone };
 struct KrylovScalars {
     double beta, om, al, omega;                     // read by every thread
     double rho, rho_new, rr, rhat2, abs_tol, r0norm, tol2;
-    int phase, restart, early, code, it, restarts, flip;
+    double rw, rr0, rw0, mix;                       // ||W r||^2, initial norms, kRestartFromStart's g
+    int phase, restart, early, code, it, restarts, flip, again;
 };
 
 // What follows a reduction: s holds its totals, q the scalars.
@@ -1010,16 +1046,27 @@ struct KrylovLimits {
     bool accept_partial;
 };
 __device__ __forceinline__ void krylov_scalars_step(KrylovScalars &q, const double (&s)[4], const KrylovLimits &lim) {
-    bool top = false, restart = false;
+    bool top = false, restart = false, back = false;
     const int phase = q.phase;
     int code = kKrylovRunning, next = kPhaseDone;
-    if (phase == kPhaseStart) {                     // ||r||^2, ||W r||^2
+    if (phase == kPhaseStart && q.again) {          // back at the start
+        q.rr = s[0];
+        q.rw = s[1];
+        q.rho_new = s[2];
+        q.rhat2 = s[3];
+        q.rho = q.al = q.omega = 1.0;
+        q.flip = 1;
+        top = true;
+    } else if (phase == kPhaseStart) {              // ||r||^2, ||W r||^2, (r_hat, r), ||r_hat||^2
         const double r0norm = sqrt(s[1]);
         const double abs_tol = fmax(lim.tol_floor, lim.inner_rtol * r0norm);
         q.r0norm = r0norm;
         q.abs_tol = abs_tol;
         q.tol2 = abs_tol * abs_tol;
-        q.rr = q.rhat2 = q.rho_new = s[0];
+        q.rr = q.rr0 = s[0];
+        q.rw = q.rw0 = s[1];
+        q.rho_new = s[2];
+        q.rhat2 = s[3];
         q.rho = q.al = q.omega = 1.0;
         q.it = q.restarts = 0;
         q.early = 0;
@@ -1054,6 +1101,7 @@ __device__ __forceinline__ void krylov_scalars_step(KrylovScalars &q, const doub
     } else {                                        // (r_hat, r), ||r||^2, ||W r||^2
         q.rho_new = s[0];
         q.rr = s[1];
+        q.rw = s[2];
         ++q.it;
         if (!isfinite(s[2])) code = kKrylovNan;
         else if (root_below(s[2], q.abs_tol, q.tol2)) code = kKrylovConverged;
@@ -1072,7 +1120,12 @@ __device__ __forceinline__ void krylov_scalars_step(KrylovScalars &q, const doub
             else code = kKrylovBreakRho;
         }
         if (stop) code = kKrylovMaxIter;
-        if (restart) {
+        back = restart && !stop && !q.again && q.rw > kRestartFromStart * q.rw0;
+        if (back) {
+            ++q.restarts;
+            q.again = 1;
+            q.mix = sqrt(q.rr0 / q.rr);
+        } else if (restart) {
             ++q.restarts;
             q.rho = 1.0; q.al = 1.0; q.omega = 1.0;
             q.rho_new = q.rr; q.rhat2 = q.rr;
@@ -1084,7 +1137,8 @@ __device__ __forceinline__ void krylov_scalars_step(KrylovScalars &q, const doub
             next = kPhaseAB;
         }
     }
-    q.restart = restart ? 1 : 0;
+    if (back) next = kPhaseStart;
+    q.restart = restart && !back ? 1 : 0;
     q.code = code;
     q.phase = code == kKrylovRunning ? next : kPhaseDone;
 }
@@ -1145,6 +1199,7 @@ __device__ __forceinline__ int krylov_slice(const KernelArgs &a, Team &g, double
         }
         ((T *)(ohm_dsmem + o.z))[R + H] = T(0);          // the padding's column
         S.phase = kPhaseStart;
+        S.again = 0;
     }
     __syncthreads();
     // On the chip the own-row vectors are one stride apart, so a row's fields
@@ -1337,8 +1392,11 @@ __device__ __forceinline__ int krylov_slice(const KernelArgs &a, Team &g, double
                 if (!spmv_long<Acc>(a, g, a.col, A, a.rowflag, z_at, row)) return kKrylovAbort;
             }
         } else {
-            // ---- start: matrix slices' values, r = r64, r_hat = r, p = v =
-            //      d = 0, preconditioner coefficients; ||r||^2, ||W r||^2 ----
+            // ---- start: matrix slices' values, r = r64, r_hat = r (again:
+            //      r64 + g r), p = v = d = 0, preconditioner coefficients;
+            //      ||r||^2, ||W r||^2, (r_hat, r), ||r_hat||^2 ----
+            const bool again = S.again != 0;
+            const double mix = S.mix;
             const uint8_t *flag = flags();
             if constexpr (MODE != kSliceCsr) {
                 const int lane = threadIdx.x & 31;
@@ -1385,15 +1443,18 @@ __device__ __forceinline__ int krylov_slice(const KernelArgs &a, Team &g, double
                 } else {
                     cs = 1.0;
                 }
+                const T rh = again ? cvt<T>(fma(mix, (double)r[li], (double)rt)) : rt;
                 p[li] = T(0);
                 v[li] = T(0);
                 r[li] = rt;
                 c[li] = cvt<T>(cs);
-                rhat[li] = rt;
+                rhat[li] = rh;
                 d[li] = 0.0;
                 if (flag[li] & kRowExport) ((KRec<T> *)a.rec0)[i] = KRec<T>{T(0), T(0), rt, cvt<T>(cs)};
                 acc[0] = fma((double)rt, (double)rt, acc[0]);
                 acc[1] = fma(wi * (double)rt, wi * (double)rt, acc[1]);
+                acc[2] = fma((double)rh, (double)rt, acc[2]);
+                acc[3] = fma((double)rh, (double)rh, acc[3]);
             }
         }
         if (!g.template reduce_then<4>(acc, [&](const double (&s)[4], bool writer) {

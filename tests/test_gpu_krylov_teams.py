@@ -126,3 +126,51 @@ def test_breakdown_at_the_iteration_limit(n, prec, max_it, restarts, code):
         assert x is None and info["status"] == _lib.ERR_SOLVE and info["krylov_code"] == code
         assert info["krylov_restarts"] == (1 + prec) * restarts
         assert info["fp64_fallbacks"] == prec
+
+
+def _source(n, spread, kind):
+    """b = e_0 with row 0 = e_0: the first iteration takes r[0] to exactly 0,
+    so (r_hat, r) = 0 and the solve restarts; column 0 (`spread` in every
+    fourth row) sets the residual it does so at.  The other rows are a
+    diagonally dominant band or 600-column mesh, for "uneven" with one row of
+    1,500 entries, for "wide" with eight entries a row."""
+    rng = np.random.default_rng(n)
+    steps = {"mesh": (1, 600), "wide": (1, 2, 5, 9)}.get(kind, (1,))
+    k = np.arange(1, n)
+    rows, cols = [], []
+    for s in steps:
+        rows += [k[k + s < n], k[k - s > 0]]
+        cols += [k[k + s < n] + s, k[k - s > 0] - s]
+    if kind == "uneven":
+        rows.append(np.full(1500, 5))
+        cols.append(10 + np.arange(1500))
+    rows, cols = np.concatenate(rows), np.concatenate(cols)
+    vals = rng.uniform(-1.0, 1.0, len(rows))
+    diag = 1.5 * np.bincount(rows, np.abs(vals), n) + 0.5
+    diag[0] = 1.0
+    far = np.arange(4, n, 4)
+    a = _csr(n, np.concatenate([rows, np.arange(n), far]), np.concatenate([cols, np.arange(n), 0 * far]),
+             np.concatenate([vals, diag, spread * diag[far]]))
+    return a, np.concatenate([[1.0], np.zeros(n - 1)])
+
+
+@pytest.mark.parametrize("spread", [0.01, 100.0], ids=["from_r", "from_start"])
+@pytest.mark.parametrize("n,kind,layouts", [(900, "band", {"chip"}), (5000, "band", {"chip"}), (40000, "band", {"chip"}),
+                                            (5000, "uneven", {"chip", "none"}), (40000, "uneven", {"chip", "none"}),
+                                            (360000, "mesh", {"stream"}), (5000, "wide", None)])
+@pytest.mark.parametrize("prec", [0, 1], ids=["fp64", "mixed"])
+def test_restart(n, kind, layouts, spread, prec):
+    """The restart from the current residual, and the one from the solve's
+    start where that residual is more than ten times the initial one.  The
+    sweeps end at ||b - A x|| < 1e-9 in FP64; x_i <= 200 puts the rounding of
+    that residual below 200 * 2^-50 * sqrt(n) = 1.1e-10."""
+    a, b = _source(n, spread, kind)
+    if layouts:
+        assert set(_layouts(a)) == layouts
+    (xs, s), (xg, g) = _solve(a, b, S.BiCgStabParams(tolerance=1e-9, max_iterations=2000, precision=prec,
+                                                     max_refinements=8))
+    assert xs is not None and s["krylov_restarts"] >= 1
+    np.testing.assert_array_equal(xs, xg)
+    assert {k: s[k] for k in ("krylov_iterations", "krylov_restarts", "fp64_fallbacks")} == \
+           {k: g[k] for k in ("krylov_iterations", "krylov_restarts", "fp64_fallbacks")}
+    assert np.linalg.norm(b - a.spmv(xs)) <= 1.2e-9
