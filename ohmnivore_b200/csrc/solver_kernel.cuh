@@ -533,7 +533,10 @@ __device__ __forceinline__ int krylov(const KernelArgs &a, Team &g, double tol_f
     out.restarts = 0;
     const bool wt = a.newton != 0;
 
-    T *rhat = (T *)a.rhat + r0, *t = (T *)a.t + r0, *d = (T *)a.d + r0;   // own rows, local index
+    T *rhat = (T *)a.rhat + r0, *t = (T *)a.t + r0;   // own rows, local index
+    // 8 bytes a row in either precision, as krylov_slice() keeps it: blocks of
+    // one team that run different forms must not overlap
+    T *d = (T *)((double *)a.d + r0);
     T *s_pair = (T *)a.s;   // s of the rows of 2x2 pairs (read by the partner in E)
     double *w = a.dx + r0;
     auto own = [&](KRec<T> *buf, int i) -> KRec<T> { return buf[i]; };

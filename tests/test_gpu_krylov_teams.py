@@ -174,3 +174,34 @@ def test_restart(n, kind, layouts, spread, prec):
     assert {k: s[k] for k in ("krylov_iterations", "krylov_restarts", "fp64_fallbacks")} == \
            {k: g[k] for k in ("krylov_iterations", "krylov_restarts", "fp64_fallbacks")}
     assert np.linalg.norm(b - a.spmv(xs)) <= 1.2e-9
+
+
+def _spilled(a, vectors, room=BLOCK_BYTES - 1024):
+    """Whether the stream layout keeps `vectors` of its eight vectors or fewer
+    in shared memory (every block)."""
+    n, blocks = a.nrows, _blocks(a.nrows)
+    r = n // blocks
+    return _up16(4 * (r // 32)) + r + 8 * r + vectors * 8 * r + 8 * r > room
+
+
+@pytest.mark.parametrize("prec", [0, 1], ids=["fp64", "mixed"])
+def test_vectors_in_global_memory_beside_the_global_solve(prec):
+    """3,600 rows a block: d (the seventh vector) and the weights leave shared
+    memory, beside one block (a row of 3,000 entries) that runs krylov(): in
+    FP32 both keep their own rows of d apart."""
+    n = 3600 * _blocks(10**6)
+    rng = np.random.default_rng(1)
+    k = np.arange(n)
+    near = [(k[k + s < n], k[k + s < n] + s) for s in (1, 600)]
+    row = n // 2 + 7
+    rows = np.concatenate([near[0][0], near[0][1], near[1][0], near[1][1], np.full(3000, row)])
+    cols = np.concatenate([near[0][1], near[0][0], near[1][1], near[1][0], row + 700 + np.arange(3000)])
+    vals = rng.uniform(-1.0, 1.0, len(rows))
+    a = _csr(n, np.concatenate([rows, k]), np.concatenate([cols, k]),
+             np.concatenate([vals, 1.2 * np.bincount(rows, np.abs(vals), n) + 0.1]))
+    kinds = _layouts(a)
+    assert kinds.count("none") == 1 and kinds.count("stream") == len(kinds) - 1 and _spilled(a, 6)
+    (xs, s), (xg, g) = _solve(a, rng.standard_normal(n), S.BiCgStabParams(tolerance=1e-12, max_iterations=500,
+                                                                          precision=prec, max_refinements=8))
+    assert xs is not None and s["krylov_iterations"] == g["krylov_iterations"]
+    np.testing.assert_array_equal(xs, xg)
