@@ -1383,7 +1383,9 @@ __device__ __forceinline__ int krylov_slice(const KernelArgs &a, Team &g, double
                 }
             }
             if (has_long) {
+                // a block alone publishes no records: z holds every row
                 auto z_at = [&](int j, bool slow) -> T {
+                    if (lone) return zvec()[j];
                     const KRec<T> q = buf[j];
                     double zz = (double)q.c * (double)u(q);
                     if (slow) {

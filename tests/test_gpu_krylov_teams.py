@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 import torch  # noqa: E402
 
-from ohmnivore_b200 import _lib, mna  # noqa: E402
+from ohmnivore_b200 import _lib, circuits as ck, mna  # noqa: E402
 from ohmnivore_b200 import solver as S  # noqa: E402
 
 BLOCK_BYTES = 227 * 1024          # shared memory of one block
@@ -205,3 +205,44 @@ def test_vectors_in_global_memory_beside_the_global_solve(prec):
                                                                           precision=prec, max_refinements=8))
     assert xs is not None and s["krylov_iterations"] == g["krylov_iterations"]
     np.testing.assert_array_equal(xs, xg)
+
+
+@pytest.mark.parametrize("prec", [0, 1], ids=["fp64", "mixed"])
+def test_long_row_in_a_team_of_one(prec):
+    """A 702-row circuit whose hub row stores each off-diagonal entry as eight
+    equal parts (5,616 entries, a long row, in one block): the same solution as
+    with each entry once, and the global-memory layout's bits."""
+    rng = np.random.default_rng(2)
+    leaves = 700
+    c = ck.CircuitBuilder()
+    c.vsource(1, 0, dc=1.0)
+    c.resistors([1], [2], [10.0])
+    leaf = 3 + np.arange(leaves)
+    c.resistors(np.full(leaves, 2), leaf, rng.uniform(1e3, 1e4, leaves))
+    c.diodes(leaf, 0, is_=1e-14, n=1.0)
+    s = mna.compile_circuit(c.build())
+    rp, hub = np.asarray(s.g.row_ptr, np.int64), s.node_index(2)
+    rows = np.repeat(np.arange(s.size), np.diff(rp))
+    parts = np.where((rows == hub) & (s.g.col != hub), 8, 1)
+    first = np.concatenate([[0], np.cumsum(parts)])
+    count = np.bincount(rows, parts, s.size).astype(np.int64)
+    many = mna.Csr(s.size, s.size, np.concatenate([[0], np.cumsum(count)]), np.repeat(s.g.col, parts),
+                   np.repeat(s.g.val / parts, parts))
+    assert count[hub] > 4096 and s.size <= 1024
+    diodes = s.diode_descriptors.copy()
+    at = diodes["g_row_col"]
+    diodes["g_row_col"] = np.where(at == mna.SENTINEL, at, first[np.minimum(at, len(parts) - 1)])
+    params = S.NewtonParams(max_iterations=100, abs_tol=1e-10, bicgstab_max_iterations=20000, bicgstab_tolerance=1e-14,
+                            precision=prec, inner_rtol=1e-4)
+    out = []
+    ctx = S.Context(0)
+    try:
+        for a, dd, layout in ((s.g, s.diode_descriptors, _lib.KRYLOV_LAYOUT_GLOBAL),
+                              (many, diodes, _lib.KRYLOV_LAYOUT_GLOBAL), (many, diodes, _lib.KRYLOV_LAYOUT_AUTO)):
+            ctx.set_krylov_layout(layout)
+            out.append(S.newton_solve(ctx, a.val, a.col, a.row_ptr, s.b_dc, dd, s.bjt_descriptors,
+                                      s.mosfet_descriptors, s.size, a.nnz, params))
+    finally:
+        ctx.close()
+    np.testing.assert_array_equal(out[1], out[2])
+    assert np.max(np.abs(out[2] - out[0])) <= 1e-9
