@@ -820,14 +820,8 @@ extern "C" ohm_status ohm_ac_sweep(ohm_ctx *c, int64_t n, int64_t nnz, const uin
     cudaLaunchAttribute cl_attr[1];
     cudaLaunchConfig_t cl_cfg = {};
     if (n >= 1) {
-        int optin = 0;
-        cudaFuncAttributes fa{};
-        if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device) == cudaSuccess &&
-            cudaFuncGetAttributes(&fa, ac_cluster_kernel) == cudaSuccess &&
-            slices.build(n, row_ptr, col, g_values, c_values, (int64_t)optin - (int64_t)fa.sharedSizeBytes - 1024,
-                         pc.partner) &&
-            cudaFuncSetAttribute(ac_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 slices.smem_bytes) == cudaSuccess &&
+        const int avail = ohm_max_dynamic_smem((const void *)ac_cluster_kernel);
+        if (avail > 0 && slices.build(n, row_ptr, col, g_values, c_values, avail, pc.partner) &&
             cudaFuncSetAttribute(ac_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
             cl_attr[0].id = cudaLaunchAttributeClusterDimension;
             cl_attr[0].val.clusterDim.x = (unsigned)slices.C;

@@ -164,6 +164,20 @@ static int choose_lpr(int64_t n, int64_t nnz) {
 
 static constexpr int kBlock = kSolverBlock;
 
+int ohm_max_dynamic_smem(const void *fn) {
+    int dev = 0, optin = 0;
+    cudaFuncAttributes fa{};
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+        cudaFuncGetAttributes(&fa, fn) != cudaSuccess)
+        return 0;
+    const int bytes = (optin - (int)fa.sharedSizeBytes - 1024) & ~15;
+    if (bytes <= 0 || (fa.maxDynamicSharedSizeBytes != bytes &&
+                       cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess))
+        return 0;
+    return bytes;
+}
+
 // Dynamic shared memory for the Krylov slice of one of `grid` blocks
 // (krylov_slice()): the chip layout with an estimate of its padded nonzeros
 // (15 % margin) and room for a halo, at most what the kernel can have; 0 when not
@@ -171,21 +185,14 @@ static constexpr int kBlock = kSolverBlock;
 // less of it there.
 static int krylov_smem_bytes(const void *fn, int64_t n, int64_t nnz_short, int grid) {
     if (n <= 0 || grid <= 0) return 0;
-    int dev = 0, optin = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
-    cudaFuncAttributes fa{};
-    if (cudaFuncGetAttributes(&fa, fn) != cudaSuccess) return 0;
-    const int64_t avail = ((int64_t)optin - (int64_t)fa.sharedSizeBytes - 1024) & ~(int64_t)15;
+    const int64_t avail = ohm_max_dynamic_smem(fn);
     const int64_t rows = (n + grid - 1) / grid + 1;
     const int64_t nnz_blk = (int64_t)((double)std::max<int64_t>(nnz_short, 0) * (double)rows / (double)n * 1.15) + 512;
     const int64_t halo = grid > 1 ? std::min<int64_t>(nnz_blk, 4096) : 0;
     const int64_t least = rows * (8 + 1) + rows / 8 + halo * 12 + 256;            // z, row flags, slice starts
     const int64_t full = least + rows * 8 * 8 + nnz_blk * (8 + 2);
     if (least > avail) return 0;
-    const int need = (int)std::min(full, avail);
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, need) != cudaSuccess) return 0;
-    return need;
+    return (int)std::min(full, avail);
 }
 
 // Grid, shared memory and synchronisation of a grid-team kernel over a

@@ -289,25 +289,21 @@ static ohm_status batch_args(ohm_batch *b, double *x_dev, const ohm_newton_param
 // largest circuit needs less.  A circuit whose slice does not fit keeps its
 // gather vector and as many of its vectors there as do (krylov_slice()).
 static int batch_smem_bytes(ohm_batch *b, BatchFn fn, int shape) {
-    int dev = 0, sm_total = 0, optin = 0;
+    int dev = 0, sm_total = 0;
     cudaFuncAttributes fa{};
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sm_total, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
         cudaFuncGetAttributes(&fa, (const void *)fn) != cudaSuccess)
         return 0;
-    const int64_t share = std::min<int64_t>(optin, sm_total / kBatchShapes[shape].min_blocks - 1024) -
-                          (int64_t)fa.sharedSizeBytes;
+    const int64_t share = std::min<int64_t>(ohm_max_dynamic_smem((const void *)fn),
+                                            sm_total / kBatchShapes[shape].min_blocks - 1024 -
+                                                (int64_t)fa.sharedSizeBytes);
     int64_t need = 0;
     for (const InstanceOffsets &o : b->h_offsets) {
         const int64_t n = o.ro1 - o.ro, z = o.no1 - o.no;
         need = std::max(need, n * (9 * 8 + 1) + n / 8 + (z + z / 4) * (8 + 2) + 512);
     }
-    const int64_t bytes = std::min(share, need) & ~(int64_t)15;
-    if (bytes <= 0 || cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)bytes) != cudaSuccess)
-        return 0;
-    return (int)bytes;
+    return (int)std::max<int64_t>(0, std::min(share, need) & ~(int64_t)15);
 }
 
 // One launch over `n` instances listed in `order` (device): a persistent grid

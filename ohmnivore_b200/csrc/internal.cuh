@@ -67,6 +67,13 @@ struct LaunchTarget {
 ohm_status ohm_launch_persistent(const LaunchTarget &t, ohm::KernelArgs &a, int64_t nnz, int *launches);
 ohm_status ohm_finish_persistent(const LaunchTarget &t, ohm_solve_info *info, int launches);
 ohm_status ohm_check_krylov(const ohm_krylov_params *p);
+// Most dynamic shared memory that a block of `fn` can have (a multiple of 16,
+// 1 KB kept free), the kernel's limit raised to it; 0 on failure.  The limit
+// belongs to the function, whatever the context or the thread: every launch
+// sets the same one, since a smaller one set by a call on another thread would
+// make a launch fail that needs more.
+int ohm_max_dynamic_smem(const void *fn);
+
 // Grid, dynamic shared memory (a.smem_bytes) and synchronisation (a.cluster)
 // of a grid-team kernel `fn` over a.n rows; `slices`: keep Krylov slices in
 // shared memory.
