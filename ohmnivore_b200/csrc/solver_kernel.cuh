@@ -211,7 +211,7 @@ enum SliceState : int {
     kSliceNone = 0,     // not built yet
     kSliceChip = 1,     // everything in shared memory
     kSliceStream = 2,   // gather vector in shared memory, matrix slices in global memory
-    kSliceCsr = 3,      // gather vector in shared memory, the CSR arrays in global memory
+    kSliceCsr = 3,      // gather vector in shared memory, the matrix in CSR form
     kSliceNo = 4,       // does not fit: global-memory solve
 };
 struct SliceMap {
@@ -837,8 +837,12 @@ namespace ohm {
 //          while they fit; the 32-row slices of the matrix in global memory,
 //          the values of as many as still fit on the chip (600 x 600 mesh,
 //          2,432 rows a block: 547 -> 537 ms);
-//   csr    (several lanes per row) vectors as in `stream`, the matrix read
-//          from its CSR arrays through local column indices;
+//   csr    (several lanes per row, or rows too uneven to pad) vectors as in
+//          `stream`; the matrix in compact rows with local column indices, on
+//          the chip where it fits.  Blocks with a few long rows: without it they
+//          ran krylov() (whole linear solves, 54 of 27,200 rows with 100 entries
+//          15.8 -> 6.8 ms, 400 of 200,000 31.5 -> 13.8 ms; 20 steps of a
+//          1,200-stage CMOS chain 61 -> 21 ms);
 //   none   z does not fit, or the halo overflows its table: krylov().
 // A block chooses for itself: blocks exchange data only through the published
 // records and the reductions (one without a slice marks every column of its
@@ -848,16 +852,16 @@ constexpr uint8_t kRowPaired = 1, kRowExport = 2, kRowLong = 4;
 
 __device__ __forceinline__ uint32_t up16(uint32_t x) { return (x + 15u) & ~15u; }
 
-// Byte offsets in dynamic shared memory: slice starts at 0, halo list, row
-// flags, columns of the matrix slices (32 W entries; none when they are in
+// Byte offsets in dynamic shared memory: slice starts at 0 (csr: the rows'
+// first nonzeros), halo list, row flags, columns of the matrix slices (32 W entries; none when they are in
 // global memory), z (R + H rows and a zero), eight own-row vectors of eight
 // bytes a row in either Krylov precision, values of the matrix slices.
 struct SliceOffsets {
     uint32_t halo, flag, col, z, vec, vec_bytes, val, end;
 };
-__device__ __forceinline__ SliceOffsets slice_offsets(uint32_t R, uint32_t H, uint32_t W) {
+__device__ __forceinline__ SliceOffsets slice_offsets(uint32_t R, uint32_t H, uint32_t W, bool csr) {
     SliceOffsets o;
-    o.halo = up16(4u * ((R + 31u) / 32u + 1u));
+    o.halo = up16(4u * ((csr ? R : (R + 31u) / 32u) + 1u));
     o.flag = o.halo + up16(4u * H);
     o.col = o.flag + up16(R);
     o.z = o.col + 64u * W;
@@ -873,6 +877,12 @@ __device__ __forceinline__ bool team_of_one(const Team &g) {
     if constexpr (std::is_same<Team, GridTeam>::value) return g.G == 1;
     else return true;
 }
+
+// Teams that can take the csr layout.  Not the one-lane kernels of a batch: a
+// third form of the solve raised their spills (944 against 564 bytes at 128
+// registers).
+template <int LPR, class Team>
+constexpr bool kHasCsr = LPR > 1 || std::is_same<Team, GridTeam>::value;
 
 // Room for the padded matrix slices of nonzeros [k0, k1) in global memory
 // (slice_val / slice_col hold 5 entries for every 4 nonzeros).
@@ -966,16 +976,20 @@ __device__ __forceinline__ bool slice_map(const KernelArgs &a, Team &g) {
     }
     const uint32_t below = room - 8u * cap;      // the table stays until the columns are known
     const uint32_t g0 = slice_start(a.row_ptr[r0]);
-    fail = fail || R + m.H >= 0xFFFF || m.W > 0xFFFF;
+    fail = fail || R + m.H >= 0xFFFF;
+    const bool pads = LPR == 1 && m.W <= 0xFFFF;        // (the offsets below fit 32 bits)
     if (!fail) {
-        const SliceOffsets chip = slice_offsets((uint32_t)R, (uint32_t)m.H, (uint32_t)m.W);
-        const SliceOffsets rest = slice_offsets((uint32_t)R, (uint32_t)m.H, 0u);
-        if (LPR == 1 && chip.end <= room && chip.z <= below) m.state = kSliceChip;
-        else if (rest.vec > room || rest.z > below || a.slice_col == nullptr) m.state = kSliceNo;
-        else if (LPR > 1) m.state = kSliceCsr;
-        else if (a.slice_val != nullptr && 32u * m.W <= slice_start(a.row_ptr[r1]) - g0) m.state = kSliceStream;
+        const SliceOffsets chip = slice_offsets((uint32_t)R, (uint32_t)m.H, pads ? (uint32_t)m.W : 0u, false);
+        const SliceOffsets rest = slice_offsets((uint32_t)R, (uint32_t)m.H, 0u, false);
+        const SliceOffsets csr = slice_offsets((uint32_t)R, (uint32_t)m.H, 0u, true);
+        if (pads && chip.end <= room && chip.z <= below) m.state = kSliceChip;
+        else if (pads && rest.vec <= room && rest.z <= below && a.slice_val != nullptr &&
+                 32u * m.W <= slice_start(a.row_ptr[r1]) - g0) m.state = kSliceStream;
+        else if (kHasCsr<LPR, Team> && csr.vec <= room && csr.z <= below && a.slice_col != nullptr)
+            m.state = kSliceCsr;
     }
-    const SliceOffsets o = slice_offsets((uint32_t)R, (uint32_t)m.H, m.state == kSliceChip ? (uint32_t)m.W : 0u);
+    const SliceOffsets o = slice_offsets((uint32_t)R, (uint32_t)m.H, m.state == kSliceChip ? (uint32_t)m.W : 0u,
+                                         m.state == kSliceCsr);
     if (m.state == kSliceNo && !lone) {
         // krylov() on this block gathers the record of every column
         for (int i = r0 + (int)threadIdx.x; i < r1; i += blockDim.x)
@@ -994,6 +1008,8 @@ __device__ __forceinline__ bool slice_map(const KernelArgs &a, Team &g) {
             return (uint16_t)(R + id[pos]);
         };
         if (m.state == kSliceCsr) {
+            // (the widths that these replace were last read before the scan)
+            for (int li = threadIdx.x; li <= R; li += blockDim.x) sl[li] = a.row_ptr[r0 + li];
             for (int li = threadIdx.x; li < R; li += blockDim.x) {
                 const uint32_t k0 = a.row_ptr[r0 + li], k1 = k0 + row_len(r0 + li);
                 for (uint32_t k = k0; k < k1; ++k) a.slice_col[k] = local(a.col[k]);
@@ -1154,7 +1170,7 @@ struct SliceView {
     void *ptr[kSliceVecs];
     const uint16_t *lcol;
     void *lval, *sval;      // stream: values of the matrix slices, the first n_sval slices on the chip
-    int n_sval;
+    int n_sval;             // csr: 1 when lcol and lval are on the chip
 };
 
 // The solve on a built slice map: a loop over phases around one reduction, so
@@ -1172,7 +1188,9 @@ __device__ __forceinline__ int krylov_slice(const KernelArgs &a, Team &g, double
     const bool pairs = g.map.pairs != 0, wt = a.newton != 0, lone = team_of_one(g), has_long = a.n_long > 0;
     const T *A;
     if constexpr (sizeof(T) == 4) A = (const T *)a.vals32; else A = (const T *)a.vals64;
-    const SliceOffsets o = slice_offsets((uint32_t)R, (uint32_t)H, MODE == kSliceChip ? (uint32_t)g.map.W : 0u);
+    const SliceOffsets o = slice_offsets((uint32_t)R, (uint32_t)H, MODE == kSliceChip ? (uint32_t)g.map.W : 0u,
+                                         MODE == kSliceCsr);
+    const uint32_t k0 = MODE == kSliceCsr ? a.row_ptr[r0] : 0u, nb = MODE == kSliceCsr ? a.row_ptr[r1] - k0 : 0u;
     if (threadIdx.x == 0) {
         if constexpr (MODE != kSliceChip) {
             // in the order of their traffic while they fit, the rest in the
@@ -1196,6 +1214,18 @@ __device__ __forceinline__ int krylov_slice(const KernelArgs &a, Team &g, double
                 const uint32_t *starts = (const uint32_t *)ohm_dsmem;
                 const uint32_t cols = at < room ? (room - at) / 256u : 0u;
                 while (fits < (R + 31) / 32 && starts[fits + 1] <= cols) ++fits;
+            }
+            if constexpr (MODE == kSliceCsr) {
+                // columns and values on the chip where both fit (both arrays
+                // are indexed by the CSR position)
+                const unsigned long long need = up16(2u * nb) + 8ull * nb;
+                if (at <= room && need <= room - at) {
+                    V_.lcol = (const uint16_t *)(ohm_dsmem + at) - k0;
+                    V_.lval = (void *)((T *)(ohm_dsmem + at + up16(2u * nb)) - k0);
+                    fits = 1;
+                } else {
+                    V_.lval = (void *)A;
+                }
             }
             V_.sval = (void *)(ohm_dsmem + at);
             V_.n_sval = fits;
@@ -1355,8 +1385,9 @@ __device__ __forceinline__ int krylov_slice(const KernelArgs &a, Team &g, double
             if constexpr (MODE == kSliceCsr) {
                 const T *z = zvec();
                 auto zx = [&](int j, bool) -> T { return z[j]; };
-                spmv_rows<LPR, Acc, T, decltype(zx), decltype(row), kRowsInFlight, false>(
-                    a.row_ptr, lcols(), A, (const uint8_t *)nullptr, r0, r1, zx, row, a.longflag);
+                spmv_rows<LPR, Acc, T, decltype(zx), decltype(row), kRowsInFlight, LPR == 1>(
+                    (const uint32_t *)ohm_dsmem, lcols(), (const T *)V.lval, (const uint8_t *)nullptr, r0, r1, zx,
+                    row, a.longflag, r0);
             } else {
                 const int lane = threadIdx.x & 31;
                 const uint32_t *sl = (const uint32_t *)ohm_dsmem;
@@ -1403,7 +1434,17 @@ __device__ __forceinline__ int krylov_slice(const KernelArgs &a, Team &g, double
             const bool again = S.again != 0;
             const double mix = S.mix;
             const uint8_t *flag = flags();
-            if constexpr (MODE != kSliceCsr) {
+            if constexpr (MODE == kSliceCsr) {
+                if (V.n_sval) {
+                    uint16_t *lc = (uint16_t *)V.lcol + k0;
+                    T *lv = (T *)V.lval + k0;
+#pragma unroll 4
+                    for (uint32_t k = threadIdx.x; k < nb; k += blockDim.x) {
+                        lc[k] = a.slice_col[k0 + k];
+                        lv[k] = A[k0 + k];
+                    }
+                }
+            } else {
                 const int lane = threadIdx.x & 31;
                 const uint32_t *sl = (const uint32_t *)ohm_dsmem;
 #pragma unroll 1
@@ -1493,8 +1534,10 @@ __device__ __forceinline__ int krylov_any(const KernelArgs &a, Team &g, double t
             return krylov_slice<T, LPR, kSliceChip>(a, g, tol_floor, inner_rtol, max_it, accept_partial, out);
         if (g.map.state == kSliceStream)
             return krylov_slice<T, LPR, kSliceStream>(a, g, tol_floor, inner_rtol, max_it, accept_partial, out);
-    } else if (g.map.state == kSliceCsr) {
-        return krylov_slice<T, LPR, kSliceCsr>(a, g, tol_floor, inner_rtol, max_it, accept_partial, out);
+    }
+    if constexpr (kHasCsr<LPR, Team>) {
+        if (g.map.state == kSliceCsr)
+            return krylov_slice<T, LPR, kSliceCsr>(a, g, tol_floor, inner_rtol, max_it, accept_partial, out);
     }
     return krylov<T, LPR>(a, g, tol_floor, inner_rtol, max_it, accept_partial, out);
 }

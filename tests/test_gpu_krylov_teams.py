@@ -1,6 +1,6 @@
 """Teams whose blocks run different forms of the Krylov solve
-(csrc/solver_kernel.cuh): a block whose slice does not fit in shared memory
-runs krylov() beside blocks that run krylov_slice().  Both have to meet at the
+(csrc/solver_kernel.cuh): a block whose nonzeros touch too many rows of other
+blocks runs krylov() beside blocks that run krylov_slice().  Both have to meet at the
 same barriers, take the same branches and give the global-memory layout's bits.
 
 ``_layouts`` restates the rule by which each block chooses, so that a test can
@@ -34,13 +34,13 @@ def _up16(b):
 
 def _layouts(a, room=BLOCK_BYTES - STATIC_BYTES):
     """Per block of a system with one lane per row and no long rows: "chip",
-    "stream" or "none" (slice_map(), slice_offsets())."""
+    "stream", "csr" or "none" (slice_map(), slice_offsets())."""
     n, blocks, rp, col = a.nrows, _blocks(a.nrows), np.asarray(a.row_ptr), np.asarray(a.col)
     assert len(col) <= 5.5 * n
     rows = -(-n // blocks) + 1
     nnz_blk = int(len(col) * rows / n * 1.15) + 512
     halo = min(nnz_blk, 4096) if blocks > 1 else 0
-    room = min(rows * 9 + rows // 8 + halo * 12 + 256 + rows * 64 + nnz_blk * 10, room) // 16 * 16
+    room = min(rows * 9 + rows // 8 + halo * 12 + 256 + rows * 68 + nnz_blk * 10, room) // 16 * 16
     bits = 0
     while 8 << (bits + 1) <= room // 2 and bits < 14:
         bits += 1
@@ -54,22 +54,24 @@ def _layouts(a, room=BLOCK_BYTES - STATIC_BYTES):
         width = np.diff(rp[r0:r1 + 1])
         w = int(sum(width[s:s + 32].max() for s in range(0, r, 32)))
 
-        def offsets(w):
-            z = _up16(4 * ((r + 31) // 32 + 1)) + _up16(4 * h) + _up16(r) + 64 * w
+        def offsets(w, starts=(r + 31) // 32):
+            z = _up16(4 * (starts + 1)) + _up16(4 * h) + _up16(r) + 64 * w
             vec = z + _up16(8 * (r + h + 1))
             return z, vec, vec + 8 * _up16(8 * r) + 256 * w
 
         z, _, end = offsets(w)
         z0, vec0, _ = offsets(0)
-        if h >= table // 4 * 3 and blocks > 1 or r + h >= 0xFFFF or w > 0xFFFF:
+        z1, vec1, _ = offsets(0, r)
+        start = lambda k: k + k // 4  # noqa: E731
+        if h >= table // 4 * 3 and blocks > 1 or r + h >= 0xFFFF:
             out.append("none")
-        elif end <= room and z <= room - 8 * table:
+        elif w <= 0xFFFF and end <= room and z <= room - 8 * table:
             out.append("chip")
-        elif vec0 > room or z0 > room - 8 * table:
-            out.append("none")
+        elif (w <= 0xFFFF and vec0 <= room and z0 <= room - 8 * table and
+              32 * w <= start(int(rp[r1])) - start(int(rp[r0]))):
+            out.append("stream")
         else:
-            start = lambda k: k + k // 4  # noqa: E731
-            out.append("stream" if 32 * w <= start(int(rp[r1])) - start(int(rp[r0])) else "none")
+            out.append("csr" if vec1 <= room and z1 <= room - 8 * table else "none")
     return out
 
 
@@ -111,14 +113,14 @@ def _skew(n, wide):
 
 @pytest.mark.parametrize("max_it,restarts,code", [(1, 1, 2), (3, 3, 2), (100, 50, 4)])
 @pytest.mark.parametrize("prec", [0, 1], ids=["fp64", "mixed"])
-@pytest.mark.parametrize("n", [4000, 30000])
+@pytest.mark.parametrize("n", [10000, 30000])
 def test_breakdown_at_the_iteration_limit(n, prec, max_it, restarts, code):
     """(r_hat, v) = 0 in every iteration: each one restarts, the last one
     allowed ends the solve (code 2), or the 51st breakdown does (code 4).  A
     block that met one barrier more or less than the others would make the call
     time out, or the FP64 solve after the failed FP32 one read partial sums that
     nobody wrote."""
-    a = _skew(n, 2000)
+    a = _skew(n, 8000)
     kinds = _layouts(a)
     assert kinds[0] == "none" and set(kinds[1:]) == {"chip"}
     params = S.BiCgStabParams(tolerance=1e-10, max_iterations=max_it, precond=_lib.PRECOND_NONE, precision=prec)
@@ -132,8 +134,8 @@ def _source(n, spread, kind):
     """b = e_0 with row 0 = e_0: the first iteration takes r[0] to exactly 0,
     so (r_hat, r) = 0 and the solve restarts; column 0 (`spread` in every
     fourth row) sets the residual it does so at.  The other rows are a
-    diagonally dominant band or 600-column mesh, for "uneven" with one row of
-    1,500 entries, for "wide" with eight entries a row."""
+    diagonally dominant band or 600-column mesh, for "uneven" and "far" with
+    one row of up to 1,500 and 8,000 entries, for "wide" with eight entries a row."""
     rng = np.random.default_rng(n)
     steps = {"mesh": (1, 600), "wide": (1, 2, 5, 9)}.get(kind, (1,))
     k = np.arange(1, n)
@@ -141,9 +143,10 @@ def _source(n, spread, kind):
     for s in steps:
         rows += [k[k + s < n], k[k - s > 0]]
         cols += [k[k + s < n] + s, k[k - s > 0] - s]
-    if kind == "uneven":
-        rows.append(np.full(1500, 5))
-        cols.append(10 + np.arange(1500))
+    if kind in ("uneven", "far"):
+        count = min(n - 20, 1500 if kind == "uneven" else 8000)
+        rows.append(np.full(count, 5))
+        cols.append(10 + np.arange(count))
     rows, cols = np.concatenate(rows), np.concatenate(cols)
     vals = rng.uniform(-1.0, 1.0, len(rows))
     diag = 1.5 * np.bincount(rows, np.abs(vals), n) + 0.5
@@ -156,7 +159,9 @@ def _source(n, spread, kind):
 
 @pytest.mark.parametrize("spread", [0.01, 100.0], ids=["from_r", "from_start"])
 @pytest.mark.parametrize("n,kind,layouts", [(900, "band", {"chip"}), (5000, "band", {"chip"}), (40000, "band", {"chip"}),
-                                            (5000, "uneven", {"chip", "none"}), (40000, "uneven", {"chip", "none"}),
+                                            (900, "uneven", {"csr"}), (5000, "uneven", {"chip", "csr"}),
+                                            (40000, "uneven", {"chip", "csr"}), (10000, "far", {"chip", "none"}),
+                                            (40000, "far", {"chip", "none"}),
                                             (360000, "mesh", {"stream"}), (5000, "wide", None)])
 @pytest.mark.parametrize("prec", [0, 1], ids=["fp64", "mixed"])
 def test_restart(n, kind, layouts, spread, prec):
@@ -187,15 +192,15 @@ def _spilled(a, vectors, room=BLOCK_BYTES - 1024):
 @pytest.mark.parametrize("prec", [0, 1], ids=["fp64", "mixed"])
 def test_vectors_in_global_memory_beside_the_global_solve(prec):
     """3,600 rows a block: d (the seventh vector) and the weights leave shared
-    memory, beside one block (a row of 3,000 entries) that runs krylov(): in
+    memory, beside one block (a row of 10,000 entries) that runs krylov(): in
     FP32 both keep their own rows of d apart."""
     n = 3600 * _blocks(10**6)
     rng = np.random.default_rng(1)
     k = np.arange(n)
     near = [(k[k + s < n], k[k + s < n] + s) for s in (1, 600)]
     row = n // 2 + 7
-    rows = np.concatenate([near[0][0], near[0][1], near[1][0], near[1][1], np.full(3000, row)])
-    cols = np.concatenate([near[0][1], near[0][0], near[1][1], near[1][0], row + 700 + np.arange(3000)])
+    rows = np.concatenate([near[0][0], near[0][1], near[1][0], near[1][1], np.full(10000, row)])
+    cols = np.concatenate([near[0][1], near[0][0], near[1][1], near[1][0], row + 700 + np.arange(10000)])
     vals = rng.uniform(-1.0, 1.0, len(rows))
     a = _csr(n, np.concatenate([rows, k]), np.concatenate([cols, k]),
              np.concatenate([vals, 1.2 * np.bincount(rows, np.abs(vals), n) + 0.1]))
