@@ -77,7 +77,8 @@ int ohm_max_dynamic_smem(const void *fn);
 // Grid, dynamic shared memory (a.smem_bytes) and synchronisation (a.cluster)
 // of a grid-team kernel `fn` over a.n rows; `slices`: keep Krylov slices in
 // shared memory.
-constexpr int kMaxTeamCluster = 16, kTeamOneBlock = 1024, kTeamRows = 512, kTeamClusterRows = 1700;
+constexpr int kMaxTeamCluster = 16, kTeamOneBlock = 1024, kTeamRows = 512, kTeamClusterRows = 1700,
+              kTeamRowNnz = 6;
 ohm_status ohm_team_shape(const void *fn, int num_sms, int max_grid, bool slices, int64_t nnz, ohm::KernelArgs &a,
                           int &grid);
 // Launch configuration of that shape: one cluster, or a cooperative grid.
