@@ -189,7 +189,8 @@ __device__ bool ac_point(const AcArgs &A, int q, AcTeam<TEAM> &g) {
     const int n = A.n, r0 = g.r0, r1 = g.r1;
     {
         const double w = A.omega[q];
-        double2 *W = A.work + (size_t)q * A.vecs * n;
+        // (a constant: with A.vecs the team kernel spilled 196 bytes, not 44)
+        double2 *W = A.work + (size_t)q * kAcVecs * n;
         double2 *x = W, *r = W + n, *rh = W + 2 * (size_t)n, *p = W + 3 * (size_t)n, *v = W + 4 * (size_t)n;
         double2 *s = W + 5 * (size_t)n, *t = W + 6 * (size_t)n, *ph = W + 7 * (size_t)n, *sh = W + 8 * (size_t)n;
         double2 *ms = W + 9 * (size_t)n, *mp = W + 10 * (size_t)n;
