@@ -686,24 +686,47 @@ __global__ void __launch_bounds__(kAcClusterBlock, 1) ac_cluster_kernel(const __
 
 using AcFn = void (*)(AcArgs);
 
-// Host side of the cluster form: per block of a cluster of C, the halo rows
-// and the 32-row matrix slices with local columns (entries filled from the G
-// and C values).
+// Host side of the cluster form: cluster size, halo rows and 32-row slices of
+// every block, and the nonzeros' local columns in CSR order.  The slices
+// themselves are filled on the device (ac_fill_slices()).
 struct AcSlices {
     int C = 0, smem_bytes = 0;
-    std::vector<uint32_t> sl_ptr, slice_base, halo_ptr, halo, pair_ptr, pair_row, pair_place, place_partner;
-    std::vector<uint16_t> col;
-    std::vector<double> g, c;
+    uint32_t entries = 0;                               // padded nonzeros / 32
+    std::vector<uint32_t> sl_ptr, sl_row, sl_end, sl_pad;   // per slice (and one more per block): entries so far,
+                                                            // its rows, the padding's column
+    std::vector<uint32_t> slice_base, halo_ptr, halo, pair_ptr, pair_row, pair_place, place_partner;
+    std::vector<uint16_t> lcol;
 
     // The smallest cluster whose blocks hold their part of a point in `avail`
-    // bytes of shared memory; false when none does.
-    bool build(int64_t n, const uint32_t *rp, const uint32_t *cl, const double *gv, const double *cv, int64_t avail,
-               const std::vector<int32_t> &partner) {
-        bool ok = false;
-        for (C = 1; C <= kAcClusterMax && !ok; ++C)
-            ok = ((n + C - 1) / C) * kAcRowBytes + 16 * 64 <= avail && fill(n, rp, cl, gv, cv, avail);
-        if (!ok) return false;
-        --C;
+    // bytes of shared memory; false when none does, or when its blocks fetch more
+    // halo rows than they own (10,000 rows of 15 scattered entries, whole calls:
+    // one point 2.0 ms in the block form, 4.0 ms so; 100 points 10.8 and 9.3;
+    // with a fifth as many halo rows as own ones 2.2 and 2.1 ms).  One pass over the
+    // nonzeros where it can be: a size is tried only when its middle block
+    // fits, and none when the middle block of the largest cluster does not
+    // (a larger cluster's blocks hold fewer rows and touch no more).
+    // (With every size tried in full and the slices filled here, the
+    // set-up of 10,000 rows of 40 entries took longer than their solve: one
+    // point 3.9 ms in the block form, 22.7 ms so.)
+    bool build(int64_t n, const uint32_t *rp, const uint32_t *cl, int64_t avail, const std::vector<int32_t> &partner,
+               bool any_pair) {
+        const int c_max = (int)std::min<int64_t>(kAcClusterMax, n);
+        std::vector<int32_t> at(n, -1);
+        lcol.resize(rp[n]);
+        C = c_max;
+        if (!start(n, avail) || !block(n, rp, cl, C / 2, avail, at)) return false;
+        const int64_t touched = (n + C - 1) / C + (int64_t)halo.size();     // a larger block touches no fewer
+        for (C = 1; C <= c_max; ++C) {
+            if (!start(n, avail)) continue;
+            if (C > 1 && touched > 2 * ((n + C - 1) / C)) return false;     // more halo rows than own ones
+            if (C > 1 && !block(n, rp, cl, C / 2, avail, at)) continue;
+            if ((int64_t)halo.size() > (n + C - 1) / C) return false;
+            start(n, avail);
+            bool ok = true;
+            for (int b = 0; b < C && ok; ++b) ok = block(n, rp, cl, b, avail, at);
+            if (ok) break;
+        }
+        if (C > c_max || (int64_t)halo.size() > n) return false;
         // halo rows and partners as places
         auto place = [&](int64_t j) -> uint32_t {
             int64_t q = (j * C) / n;
@@ -712,10 +735,10 @@ struct AcSlices {
         };
         for (uint32_t &h : halo) h = place(h) | (partner[h] >= 0 ? kPlacePaired : 0u);
         pair_ptr.assign(1, 0);
-        place_partner.assign(n, 0);
+        if (any_pair) place_partner.assign(n, 0);
         for (int b = 0; b < C; ++b) {
             const int64_t r0 = n * b / C, r1 = n * (b + 1) / C;
-            for (int64_t i = r0; i < r1; ++i) {
+            for (int64_t i = any_pair ? r0 : r1; i < r1; ++i) {
                 if (partner[i] < 0) continue;
                 place_partner[i] = place(partner[i]);
                 pair_row.push_back((uint32_t)(i - r0));
@@ -725,54 +748,78 @@ struct AcSlices {
         }
         return true;
     }
-    bool fill(int64_t n, const uint32_t *rp, const uint32_t *cl, const double *gv, const double *cv, int64_t avail) {
-        const int64_t stride = (n + C - 1) / C, nnz = rp[n];
-        std::vector<int32_t> at(n, -1);
-        sl_ptr.clear(); slice_base.clear(); halo.clear(); col.clear(); g.clear(); c.clear();
+
+private:
+    bool start(int64_t n, int64_t avail) {
+        sl_ptr.clear(); sl_row.clear(); sl_end.clear(); sl_pad.clear(); slice_base.clear(); halo.clear();
         halo_ptr.assign(1, 0);
-        uint32_t w_total = 0;
-        size_t h_max = 0;
-        for (int b = 0; b < C; ++b) {
-            const int64_t r0 = n * b / C, r1 = n * (b + 1) / C, R = r1 - r0;
-            const size_t h0 = halo.size();
-            for (uint32_t k = rp[r0]; k < rp[r1]; ++k) {
-                const int64_t j = cl[k];
-                if ((j >= r0 && j < r1) || at[j] >= 0) continue;
+        entries = 0;
+        smem_bytes = 0;
+        return ((n + C - 1) / C) * kAcRowBytes + 16 * 64 <= avail;
+    }
+    // Appends block b; false when it does not fit.  at: -1 everywhere, and again afterwards.
+    bool block(int64_t n, const uint32_t *rp, const uint32_t *cl, int b, int64_t avail, std::vector<int32_t> &at) {
+        const int64_t r0 = n * b / C, r1 = n * (b + 1) / C, R = r1 - r0, stride = (n + C - 1) / C;
+        const size_t h0 = halo.size();
+        // 16 bytes of z and 4 of its place for a halo row, and a zero
+        const int64_t h_fit = std::min<int64_t>((avail - stride * kAcRowBytes - 32) / 20, 0xFFFE - R);
+        bool ok = true;
+        for (uint32_t k = rp[r0]; k < rp[r1] && ok; ++k) {
+            const int64_t j = cl[k];
+            if (j >= r0 && j < r1) {
+                lcol[k] = (uint16_t)(j - r0);
+                continue;
+            }
+            if (at[j] < 0) {
+                ok = (int64_t)(halo.size() - h0) < h_fit;
                 at[j] = (int32_t)(R + (int64_t)(halo.size() - h0));
                 halo.push_back((uint32_t)j);
             }
-            const size_t H = halo.size() - h0;
-            h_max = std::max(h_max, H);
-            if (R + (int64_t)H >= 0xFFFF) return false;
-            slice_base.push_back((uint32_t)sl_ptr.size());
-            for (int64_t s = r0; s < r1; s += 32) {
-                uint32_t width = 0;
-                for (int64_t i = s; i < std::min(r1, s + 32); ++i) width = std::max(width, rp[i + 1] - rp[i]);
-                sl_ptr.push_back(w_total);
-                w_total += width;
-                if (32ull * w_total > 2ull * (uint64_t)nnz + 4096) return false;    // rows too uneven to pad
-                const size_t e0 = g.size();
-                g.resize(e0 + 32ull * width, 0.0);
-                c.resize(e0 + 32ull * width, 0.0);
-                col.resize(e0 + 32ull * width, (uint16_t)(R + (int64_t)H));
-                for (int64_t i = s; i < std::min(r1, s + 32); ++i)
-                    for (uint32_t k = rp[i]; k < rp[i + 1]; ++k) {
-                        const size_t e = e0 + 32ull * (k - rp[i]) + (size_t)(i - s);
-                        const int64_t j = cl[k];
-                        g[e] = gv[k];
-                        c[e] = cv ? cv[k] : 0.0;
-                        col[e] = (uint16_t)(j >= r0 && j < r1 ? j - r0 : at[j]);
-                    }
-            }
-            sl_ptr.push_back(w_total);
-            for (size_t h = h0; h < halo.size(); ++h) at[halo[h]] = -1;
-            halo_ptr.push_back((uint32_t)halo.size());
+            lcol[k] = (uint16_t)at[j];
         }
-        const int64_t bytes = stride * kAcRowBytes + 16 * ((int64_t)h_max + 1) + 4 * (int64_t)h_max + 16;
-        smem_bytes = (int)bytes;
-        return bytes <= avail;
+        for (size_t h = h0; h < halo.size(); ++h) at[halo[h]] = -1;
+        const int64_t H = (int64_t)(halo.size() - h0);
+        halo_ptr.push_back((uint32_t)halo.size());
+        slice_base.push_back((uint32_t)sl_ptr.size());
+        for (int64_t s = r0; s < r1 && ok; s += 32) {
+            uint32_t width = 0;
+            for (int64_t i = s; i < std::min(r1, s + 32); ++i) width = std::max(width, rp[i + 1] - rp[i]);
+            slice(s, std::min(r1, s + 32), R + H);
+            entries += width;
+            ok = 32ull * entries <= 2ull * (uint64_t)rp[n] + 4096;      // else rows too uneven to pad
+        }
+        slice(r1, r1, R + H);
+        smem_bytes = std::max(smem_bytes, (int)(stride * kAcRowBytes + 20 * H + 32));
+        return ok;
+    }
+    void slice(int64_t row, int64_t end, int64_t pad) {
+        sl_ptr.push_back(entries);
+        sl_row.push_back((uint32_t)row);
+        sl_end.push_back((uint32_t)end);
+        sl_pad.push_back((uint32_t)pad);
     }
 };
+
+// Fills the matrix slices from the CSR arrays: one warp a slice, its lanes the
+// slice's rows.  Padding has value 0 and the column of a zero.
+__global__ void ac_fill_slices(int n_slices, const uint32_t *__restrict__ sl_ptr, const uint32_t *__restrict__ sl_row,
+                               const uint32_t *__restrict__ sl_end, const uint32_t *__restrict__ sl_pad,
+                               const uint32_t *__restrict__ rp, const uint16_t *__restrict__ lcol,
+                               const double *__restrict__ g, const double *__restrict__ c, uint16_t *col, double *gval,
+                               double *cval) {
+    const int s = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (s >= n_slices || sl_row[s] == sl_end[s]) return;       // (a block's last entry has no rows)
+    const uint32_t i = sl_row[s] + lane, end = sl_end[s], pad = sl_pad[s], e0 = sl_ptr[s];
+    const uint32_t width = sl_ptr[s + 1] - e0;
+    const uint32_t k0 = i < end ? rp[i] : 0u, len = i < end ? rp[i + 1] - k0 : 0u;
+    for (uint32_t k = 0; k < width; ++k) {
+        const size_t e = (size_t)(e0 + k) * 32 + lane;
+        const bool in = k < len;
+        col[e] = in ? lcol[k0 + k] : (uint16_t)pad;
+        gval[e] = in ? g[k0 + k] : 0.0;
+        if (c) cval[e] = in ? c[k0 + k] : 0.0;
+    }
+}
 
 AcFn pick_ac(double avg, bool wide) {
     if (wide) {
@@ -817,12 +864,13 @@ extern "C" ohm_status ohm_ac_sweep(ohm_ctx *c, int64_t n, int64_t nnz, const uin
     // cluster form where a point fits a cluster's shared memory
     AcSlices slices;
     AcClusterArgs K{};
+    std::vector<uint32_t> words;
     int clusters = 0;
     cudaLaunchAttribute cl_attr[1];
     cudaLaunchConfig_t cl_cfg = {};
     if (n >= 1) {
         const int avail = ohm_max_dynamic_smem((const void *)ac_cluster_kernel);
-        if (avail > 0 && slices.build(n, row_ptr, col, g_values, c_values, avail, pc.partner) &&
+        if (avail > 0 && slices.build(n, row_ptr, col, avail, pc.partner, pc.any_pair) &&
             cudaFuncSetAttribute(ac_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
             cl_attr[0].id = cudaLaunchAttributeClusterDimension;
             cl_attr[0].val.clusterDim.x = (unsigned)slices.C;
@@ -882,20 +930,34 @@ extern "C" ohm_status ohm_ac_sweep(ohm_ctx *c, int64_t n, int64_t nnz, const uin
         K.C = slices.C;
         K.smem_bytes = slices.smem_bytes;
         K.any_pair = pc.any_pair ? 1 : 0;
+        // the index arrays as one upload
+        const std::vector<uint32_t> *parts[] = {&slices.sl_ptr,   &slices.sl_row, &slices.sl_end,   &slices.sl_pad,
+                                                &slices.slice_base, &slices.halo_ptr, &slices.halo, &slices.pair_ptr,
+                                                &slices.pair_row, &slices.pair_place, &slices.place_partner};
+        size_t first[11];
+        for (int q = 0; q < 11; ++q) {
+            first[q] = words.size();
+            words.insert(words.end(), parts[q]->begin(), parts[q]->end());
+        }
         uint32_t *u = nullptr;
-        uint16_t *h = nullptr;
-        double *d = nullptr;
-        if (e == cudaSuccess) { e = put(&u, slices.sl_ptr.data(), slices.sl_ptr.size()); K.sl_ptr = u; }
-        if (e == cudaSuccess) { e = put(&u, slices.slice_base.data(), slices.slice_base.size()); K.slice_base = u; }
-        if (e == cudaSuccess) { e = put(&u, slices.halo_ptr.data(), slices.halo_ptr.size()); K.halo_ptr = u; }
-        if (e == cudaSuccess) { e = put(&u, slices.halo.data(), slices.halo.size()); K.halo = u; }
-        if (e == cudaSuccess) { e = put(&u, slices.pair_ptr.data(), slices.pair_ptr.size()); K.pair_ptr = u; }
-        if (e == cudaSuccess) { e = put(&u, slices.pair_row.data(), slices.pair_row.size()); K.pair_row = u; }
-        if (e == cudaSuccess) { e = put(&u, slices.pair_place.data(), slices.pair_place.size()); K.pair_place = u; }
-        if (e == cudaSuccess) { e = put(&u, slices.place_partner.data(), slices.place_partner.size()); K.place_partner = u; }
-        if (e == cudaSuccess) { e = put(&h, slices.col.data(), slices.col.size()); K.col = h; }
-        if (e == cudaSuccess) { e = put(&d, slices.g.data(), slices.g.size()); K.gval = d; }
-        if (e == cudaSuccess && c_values) { e = put(&d, slices.c.data(), slices.c.size()); K.cval = d; }
+        uint16_t *lc = nullptr, *h = nullptr;
+        double *gv = nullptr, *cv = nullptr;
+        const size_t padded = 32 * (size_t)slices.entries;
+        if (e == cudaSuccess) e = put(&u, words.data(), words.size());
+        if (e == cudaSuccess) e = put(&lc, slices.lcol.data(), slices.lcol.size());
+        if (e == cudaSuccess) e = put(&h, (const uint16_t *)nullptr, padded);
+        if (e == cudaSuccess) e = put(&gv, (const double *)nullptr, padded);
+        if (e == cudaSuccess && c_values) e = put(&cv, (const double *)nullptr, padded);
+        K.sl_ptr = u + first[0]; K.slice_base = u + first[4]; K.halo_ptr = u + first[5]; K.halo = u + first[6];
+        K.pair_ptr = u + first[7]; K.pair_row = u + first[8]; K.pair_place = u + first[9];
+        K.place_partner = u + first[10];
+        K.col = h; K.gval = gv; K.cval = cv;
+        if (e == cudaSuccess) {
+            const int n_slices = (int)slices.sl_ptr.size();
+            ac_fill_slices<<<(n_slices + 7) / 8, 256, 0, c->stream>>>(n_slices, K.sl_ptr, u + first[1], u + first[2],
+                                                                      u + first[3], d_rp, lc, d_g, d_c, h, gv, cv);
+            e = cudaGetLastError();
+        }
     }
     // a point per SM at most: give each point a whole SM when the system is large
     const bool wide = n >= 2048 && n_freq <= c->num_sms;
