@@ -143,7 +143,7 @@ extern "C" ohm_status ohm_ctx_set_krylov_layout(ohm_ctx *c, int32_t layout) {
 }
 
 // ------------------------------------------------------------ launch logic --
-static KernelFn pick_kernel(int lpr) {
+static KernelPair<KernelFn> pick_kernel(int lpr) {
     switch (lpr) {
         case 1: return persistent_kernel_for<1>();
         case 4: return persistent_kernel_for<4>();
@@ -162,8 +162,6 @@ static int choose_lpr(int64_t n, int64_t nnz) {
     return 32;
 }
 
-static constexpr int kBlock = kSolverBlock;
-
 int ohm_max_dynamic_smem(const void *fn) {
     int dev = 0, optin = 0;
     cudaFuncAttributes fa{};
@@ -181,13 +179,12 @@ int ohm_max_dynamic_smem(const void *fn) {
 // Dynamic shared memory for the Krylov slice of one of `grid` blocks
 // (krylov_slice()): the chip layout with an estimate of its padded nonzeros
 // (15 % margin, as much as the compact rows of the csr layout take) and room for a
-// halo, at most what the kernel can have; 0 when not even the gather vector
-// fits.  Not always the most: what it leaves is L1, which the passes outside
+// halo, at most `avail`, what the kernel can have; 0 when not even the gather
+// vector fits.  Not always the most: what it leaves is L1, which the passes outside
 // the Krylov solve need (all of it requested: 401-row transient 39.0 -> 41.6
 // ms, 100,000-stage chain 24.7 -> 25.7 ms, ISAI(1) of 400 rows 0.91 -> 1.31 ms).
-static int krylov_smem_bytes(const void *fn, int64_t n, int64_t nnz_short, int grid) {
+static int krylov_smem_bytes(int64_t avail, int64_t n, int64_t nnz_short, int grid) {
     if (n <= 0 || grid <= 0) return 0;
-    const int64_t avail = ohm_max_dynamic_smem(fn);
     const int64_t rows = (n + grid - 1) / grid + 1;
     const int64_t nnz_blk = (int64_t)((double)std::max<int64_t>(nnz_short, 0) * (double)rows / (double)n * 1.15) + 512;
     const int64_t halo = grid > 1 ? std::min<int64_t>(nnz_blk, 4096) : 0;
@@ -196,8 +193,8 @@ static int krylov_smem_bytes(const void *fn, int64_t n, int64_t nnz_short, int g
     return least > avail ? 0 : (int)std::min(full & ~(int64_t)15, avail);
 }
 
-// Grid, shared memory and synchronisation of a grid-team kernel over a
-// system of a.n rows, by the larger of its rows and devices:
+// Blocks of a grid team over a system of n rows, by the larger of its rows and
+// devices:
 //   up to 1,024: one block, which needs no team barrier (401- and 578-row
 //     systems on two blocks: +22 %);
 //   then one block per 512, as one cluster of up to 16 blocks (its barrier
@@ -206,41 +203,93 @@ static int krylov_smem_bytes(const void *fn, int64_t n, int64_t nnz_short, int g
 //     BiCGSTAB iteration 1,602 rows 10.4 -> 9.3 us, 3,602 rows 10.2 -> 9.1
 //     against one block per 1,024; 22,502 rows on 16 blocks 11.4 us, on a grid
 //     of 22 13.6 us;
-//   beyond: one block per 512, at most one per SM (27,227 rows 13.3 -> 12.2
-//     us).
+//   beyond, and where a cluster's blocks reach too far (ohm_scatter()): one
+//     block per 512, at most one per SM (27,227 rows 13.3 -> 12.2 us).
 // Above one block, six nonzeros count as a row, so that systems of several
 // lanes a row get the blocks that their products want (whole solves, by rows
 // alone -> so: 27,000 rows of 9 random entries 2.32 -> 1.19 ms, 20,000 of 31
 // 3.27 -> 1.74, 5,000 of 41 0.92 -> 0.71).
-ohm_status ohm_team_shape(const void *fn, int num_sms, int max_grid, bool slices, int64_t nnz, KernelArgs &a,
-                          int &grid) {
+static int team_blocks(int64_t n, int64_t n_devices, int64_t nnz, bool cluster, int64_t cap) {
+    int64_t items = std::max(n, n_devices);
+    if (items <= kTeamOneBlock) return 1;
+    items = std::max(items, nnz / kTeamRowNnz);
+    int64_t want = (items + kTeamRows - 1) / kTeamRows;
+    if (cluster && items <= kMaxTeamCluster * kTeamClusterRows) want = std::min<int64_t>(want, kMaxTeamCluster);
+    return (int)std::max<int64_t>(1, std::min(want, cap));
+}
+
+// A cluster is left where its blocks share more than kClusterReach columns with
+// others: a phase then waits for more than six records a thread one after the
+// other (25,600-row mesh in random order, 16 blocks -> 50: 27 -> 14 us per
+// iteration; 10,000 rows, 2,400 columns: 12.1 us on 16).
+constexpr int64_t kClusterReach = 3072;
+
+// Three blocks of the team are looked at; the answer is that of two of them.
+// (A block that reaches too far although the others do not runs krylov() beside
+// them.)
+int ohm_scatter(int64_t n, int64_t n_devices, int num_sms, const uint32_t *rp, const uint32_t *col) {
+    if (std::max(n, n_devices) <= kTeamOneBlock) return kScatterNear;
+    std::vector<uint8_t> seen((size_t)n, 0);
+    uint8_t mark = 0;
+    auto near = [&](int grid) {
+        const int smem = krylov_smem_bytes((227 << 10) - 4096, n, rp[n], grid);
+        int64_t table = 1;                             // slots of the halo table (slice_map())
+        while (16 * table <= smem / 2 && table < (1 << 14)) table *= 2;
+        int fits = 0;
+        for (int q = 1; q <= 3; ++q) {
+            const int64_t b = (int64_t)grid * q / 4, r0 = n * b / grid, r1 = n * (b + 1) / grid;
+            int64_t reach = 0;
+            ++mark;
+            for (int64_t i = r0; i < r1; ++i) {
+                if (rp[i + 1] - rp[i] > kLongRowMin) continue;
+                for (uint32_t k = rp[i]; k < rp[i + 1]; ++k) {
+                    const int64_t j = col[k];
+                    if ((j >= r0 && j < r1) || seen[j] == mark) continue;
+                    seen[j] = mark;
+                    ++reach;
+                }
+            }
+            if (reach < (grid <= kMaxTeamCluster ? std::min(table / 4 * 3, kClusterReach) : table / 4 * 3)) ++fits;
+        }
+        return fits >= 2;
+    };
+    const int grid = team_blocks(n, n_devices, rp[n], true, num_sms);
+    if (near(grid)) return kScatterNear;
+    const int all = team_blocks(n, n_devices, rp[n], false, num_sms);
+    return all > grid && near(all) ? kScatterWide : kScatterFar;
+}
+
+ohm_status ohm_team_shape(const void *slices, const void *wide, int num_sms, int max_grid, int krylov_layout,
+                          int64_t nnz, KernelArgs &a, TeamShape &s) {
+    const bool automatic = krylov_layout != OHM_KRYLOV_LAYOUT_GLOBAL, isai = a.precond == kPcIsai;
+    const int scatter = automatic && !isai ? a.scatter : kScatterNear;
+    const int64_t cap = max_grid > 0 ? std::min(num_sms, max_grid) : num_sms;
+    const int64_t nnz_short = nnz - a.nnz_long;
+    s = TeamShape{};
+    s.grid = team_blocks(a.n, (int64_t)a.nd + a.nq + a.nm, nnz_short, scatter == kScatterNear, cap);
+    a.smem_bytes = automatic && !isai && a.slice_export && scatter != kScatterFar
+                       ? krylov_smem_bytes(ohm_max_dynamic_smem(slices), a.n, nnz_short, s.grid) : 0;
+    // the global-memory form of large systems, unless the caller asked for it
+    // (OHM_KRYLOV_LAYOUT_GLOBAL gives the bits of the slices)
+    s.wide = automatic && a.smem_bytes == 0 && s.grid > kMaxTeamCluster;
+    const void *fn = s.wide ? wide : slices;
+    s.block = s.wide ? kWideBlock : kSolverBlock;
     int per_sm = 0;
-    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kBlock, 0));
-    if (per_sm < 1) return fail(OHM_ERR_CUDA, "solver kernel does not fit on an SM");
-    int64_t items = std::max<int64_t>(a.n, (int64_t)a.nd + a.nq + a.nm);
-    const bool one = items <= kTeamOneBlock;
-    items = std::max(items, (nnz - a.nnz_long) / kTeamRowNnz);
-    int64_t want = one ? 1 : (items + kTeamRows - 1) / kTeamRows;
-    if (items <= kMaxTeamCluster * kTeamClusterRows) want = std::min<int64_t>(want, kMaxTeamCluster);
-    int64_t cap = num_sms;
-    if (max_grid > 0) cap = std::min<int64_t>(cap, max_grid);
-    grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, cap));
-    a.smem_bytes = slices && a.slice_export ? krylov_smem_bytes(fn, a.n, nnz - a.nnz_long, grid) : 0;
-    if (a.smem_bytes > 0) {
-        int fit = 0;
-        CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, fn, kBlock, a.smem_bytes));
-        if (fit < 1) a.smem_bytes = 0;
-        else grid = (int)std::min<int64_t>(grid, (int64_t)fit * num_sms);
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, s.block, a.smem_bytes));
+    if (per_sm < 1 && a.smem_bytes > 0) {
+        a.smem_bytes = 0;
+        CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, s.block, 0));
     }
+    if (per_sm < 1) return fail(OHM_ERR_CUDA, "solver kernel does not fit on an SM");
     a.cluster = 0;
-    if (grid >= 2 && grid <= kMaxTeamCluster) {
+    if (s.grid >= 2 && s.grid <= kMaxTeamCluster) {
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = grid;
+        attr[0].val.clusterDim.x = s.grid;
         attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        cfg.gridDim = dim3(grid);
-        cfg.blockDim = dim3(kBlock);
+        cfg.gridDim = dim3(s.grid);
+        cfg.blockDim = dim3(s.block);
         cfg.dynamicSmemBytes = (size_t)a.smem_bytes;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
@@ -255,18 +304,17 @@ ohm_status ohm_team_shape(const void *fn, int num_sms, int max_grid, bool slices
 }
 
 ohm_status ohm_launch_persistent(const LaunchTarget &t, KernelArgs &a, int64_t nnz, int *launches) {
-    const int lpr = choose_lpr(a.n, nnz);
-    KernelFn fn = pick_kernel(lpr);
-    int grid = 0;
-    const ohm_status st = ohm_team_shape((const void *)fn, t.num_sms, t.max_grid,
-                                         t.krylov_layout != OHM_KRYLOV_LAYOUT_GLOBAL, nnz, a, grid);
+    TeamShape shape;
+    KernelFn fn = nullptr;
+    const ohm_status st = ohm_team_kernel(pick_kernel(choose_lpr(a.n, nnz)), t.num_sms, t.max_grid, t.krylov_layout,
+                                          nnz, a, shape, fn);
     if (st != OHM_OK) return st;
     a.gs.count = (unsigned long long *)t.sync_words;     // words 0-1
     a.gs.error = (int *)(t.sync_words + 2);              // word 2
     a.info = t.info_dev;
     CUDA_TRY(cudaMemsetAsync(t.sync_words, 0, 4 * sizeof(unsigned int), t.stream));
     CUDA_TRY(cudaMemsetAsync(t.info_dev, 0, sizeof(DeviceInfo), t.stream));
-    TeamLaunch cfg(grid, a, t.stream);
+    TeamLaunch cfg(shape, a, t.stream);
     CUDA_TRY(cudaLaunchKernelEx(&cfg.config, fn, a));
     if (launches) *launches += 1;
     return OHM_OK;
@@ -352,6 +400,7 @@ struct Workspace {
     double *slice_val = nullptr;
     uint8_t *slice_export = nullptr;
     bool any_pair = false;
+    int scatter = kScatterNear;
     void release() {
         ohm_pool_free(vec); ohm_pool_free(r64); ohm_pool_free(dx); ohm_pool_free(partials);
         ohm_pool_free(partner); ohm_pool_free(diag_slot); ohm_pool_free(off_slot); ohm_pool_free(rowflag);
@@ -383,6 +432,7 @@ struct Workspace {
         a.slice_col = slice_col;
         a.slice_val = slice_val;
         a.slice_export = slice_export;
+        a.scatter = scatter;
         a.r64 = r64;
         a.dx = dx;
         a.partials = partials;
@@ -508,6 +558,7 @@ static ohm_status solve_real_impl(ohm_ctx *c, int64_t n, int64_t nnz, const uint
     PcHost pc;
     build_precond(n, h_rp, h_col, h_val, {}, p->precond == OHM_PRECOND_AUTO, pc);
     e = ws.upload_pc(pc, c->stream);
+    ws.scatter = ohm_scatter(n, 0, c->num_sms, h_rp, h_col);
     IsaiDev isai;
     if (e == cudaSuccess && p->precond == OHM_PRECOND_ISAI1) e = isai.build(n, h_rp, h_col, c->stream);
     if (e == cudaSuccess && mixed && nnz > 0) {
@@ -743,6 +794,7 @@ extern "C" ohm_status ohm_plan_create(ohm_ctx *c, const double *base_g_values, c
     bool host_ok = true;
     try {
         sflag = stamp_flags(size, row_ptrs, col_indices, p->touched, rs);
+        p->ws.scatter = ohm_scatter(size, n_diodes + n_bjts + n_mosfets, c->num_sms, row_ptrs, col_indices);
         split_long(size, row_ptrs, kLongRowMin, kLongRowChunk, 0, lrows);
         split_long((int64_t)ms.size(), mptr.data(), kLongSegMin, kLongSegChunk, 0, lsegs);
         split_long((int64_t)rs.size(), rptr.data(), kLongSegMin, kLongSegChunk, (int64_t)ms.size(), lsegs);
@@ -1196,6 +1248,7 @@ ohm_status ohm_linsys_create(ohm_ctx *c, int64_t n, int64_t nnz, const uint32_t 
     if (e == cudaSuccess) e = dalloc(&L->col, nnz);
     if (e == cudaSuccess) e = cudaMemcpyAsync(L->rp, h_rp, (n + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess && nnz) e = cudaMemcpyAsync(L->col, h_col, nnz * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream);
+    L->ws.scatter = ohm_scatter(n, 0, c->num_sms, h_rp, h_col);
     if (e == cudaSuccess) e = L->ws.alloc(n, nnz, c->num_sms);
     if (e == cudaSuccess) e = L->ws.upload_pc(pc, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);

@@ -32,6 +32,7 @@ struct ohm_batch {
     // Host copies of the offset tables and of the largest-first order, for
     // instances solved one at a time by the whole GPU (ohm_batch_set_split).
     std::vector<InstanceOffsets> h_offsets;
+    std::vector<int8_t> scatter;        // per instance (ohm_scatter())
     std::vector<int32_t> h_order;
     double *team_partials = nullptr;   // reduction partials of those solves
     int split = 1;
@@ -78,6 +79,7 @@ extern "C" ohm_status ohm_batch_create(ohm_ctx *c, int64_t n_inst, const int64_t
     std::vector<int32_t> partner(rows);
     std::vector<uint32_t> diag(rows), off(rows);
     std::vector<uint8_t> flag(rows), sflag(rows);
+    std::vector<int8_t> scatter(n_inst, kScatterNear);
     bool any_pair = false;
     int64_t max_nnz_row = 0;
     for (int64_t i = 0; i < n_inst; ++i) {
@@ -135,6 +137,7 @@ extern "C" ohm_status ohm_batch_create(ohm_ctx *c, int64_t n_inst, const int64_t
         std::copy(pc.off_slot.begin(), pc.off_slot.end(), off.begin() + row_off[i]);
         std::copy(pc.rowflag.begin(), pc.rowflag.end(), flag.begin() + row_off[i]);
         any_pair |= pc.any_pair;
+        scatter[i] = (int8_t)ohm_scatter(n, dn + qn + mn, c->num_sms, rp, cl);
         for (int64_t r = 0; r < n; ++r) max_nnz_row = std::max<int64_t>(max_nnz_row, rp[r + 1] - rp[r]);
     }
     // longest first
@@ -224,6 +227,7 @@ extern "C" ohm_status ohm_batch_create(ohm_ctx *c, int64_t n_inst, const int64_t
     b->args.queue = b->queue;
     b->host_infos.resize(n_inst);
     b->h_order = order;
+    b->scatter = scatter;
     b->h_offsets.resize(n_inst);
     for (int64_t i = 0; i < n_inst; ++i) {
         InstanceOffsets &o = b->h_offsets[i];
@@ -368,6 +372,7 @@ static ohm_status solve_instance_whole_gpu(ohm_batch *b, const BatchArgs &B, int
     ohm_ctx *c = b->ctx;
     KernelArgs a;
     instance_args(B, i, b->h_offsets[i], a);
+    a.scatter = b->scatter[i];
     a.partials = b->team_partials;
     const LaunchTarget t{c->num_sms, c->stream, c->sync_words, c->info_dev, c->info_host, 0, c->krylov_layout};
     ohm_status st = ohm_launch_persistent(t, a, a.nnz, launches);

@@ -12,20 +12,27 @@
 
 using ohm::DeviceInfo;
 
+// A grid-team kernel with Krylov slices (kSolverBlock threads) and its
+// global-memory form (kWideBlock threads).
+template <typename Fn>
+struct KernelPair {
+    Fn slices, wide;
+};
+
 // The persistent solver per lanes per row, instantiated in solver_k*.cu.
 using KernelFn = void (*)(ohm::KernelArgs);
 template <int LPR>
-KernelFn persistent_kernel_for();
+KernelPair<KernelFn> persistent_kernel_for();
 template <>
-KernelFn persistent_kernel_for<1>();
+KernelPair<KernelFn> persistent_kernel_for<1>();
 template <>
-KernelFn persistent_kernel_for<4>();
+KernelPair<KernelFn> persistent_kernel_for<4>();
 template <>
-KernelFn persistent_kernel_for<8>();
+KernelPair<KernelFn> persistent_kernel_for<8>();
 template <>
-KernelFn persistent_kernel_for<16>();
+KernelPair<KernelFn> persistent_kernel_for<16>();
 template <>
-KernelFn persistent_kernel_for<32>();
+KernelPair<KernelFn> persistent_kernel_for<32>();
 
 // Records the message for ohm_last_error() and returns `st`.
 ohm_status ohm_fail(ohm_status st, const char *fmt, ...);
@@ -74,25 +81,47 @@ ohm_status ohm_check_krylov(const ohm_krylov_params *p);
 // make a launch fail that needs more.
 int ohm_max_dynamic_smem(const void *fn);
 
-// Grid, dynamic shared memory (a.smem_bytes) and synchronisation (a.cluster)
-// of a grid-team kernel `fn` over a.n rows; `slices`: keep Krylov slices in
-// shared memory.
+// How far the rows of a system's blocks reach, from its pattern on the host:
+// kScatterNear when the columns that a block shares with others fit its halo
+// table (krylov_slice()), kScatterWide when they do so with one block per
+// kTeamRows rows but not in a cluster of kMaxTeamCluster, kScatterFar when they
+// do not: such a system (rows in random order, a random graph) runs krylov() in
+// every block, which wants its shared memory as L1 and 1,024 threads (us per
+// iteration with 512 threads that reserved a slice -> so: 500 x 500 mesh in
+// random order 54 -> 35, 700 x 700 91 -> 55, 1000 x 1000 243 -> 117).
+enum Scatter : int { kScatterNear = 0, kScatterWide = 1, kScatterFar = 2 };
+int ohm_scatter(int64_t n, int64_t n_devices, int num_sms, const uint32_t *row_ptr, const uint32_t *col);
+
+// Grid, block, kernel form, dynamic shared memory (a.smem_bytes) and
+// synchronisation (a.cluster) of a grid-team kernel over a.n rows.
 constexpr int kMaxTeamCluster = 16, kTeamOneBlock = 1024, kTeamRows = 512, kTeamClusterRows = 1700,
               kTeamRowNnz = 6;
-ohm_status ohm_team_shape(const void *fn, int num_sms, int max_grid, bool slices, int64_t nnz, ohm::KernelArgs &a,
-                          int &grid);
+struct TeamShape {
+    int grid = 1, block = ohm::kSolverBlock;
+    bool wide = false;
+};
+ohm_status ohm_team_shape(const void *slices, const void *wide, int num_sms, int max_grid, int krylov_layout,
+                          int64_t nnz, ohm::KernelArgs &a, TeamShape &s);
+template <typename Fn>
+ohm_status ohm_team_kernel(const KernelPair<Fn> &k, int num_sms, int max_grid, int krylov_layout, int64_t nnz,
+                           ohm::KernelArgs &a, TeamShape &s, Fn &fn) {
+    const ohm_status st = ohm_team_shape((const void *)k.slices, (const void *)k.wide, num_sms, max_grid,
+                                         krylov_layout, nnz, a, s);
+    fn = s.wide ? k.wide : k.slices;
+    return st;
+}
 // Launch configuration of that shape: one cluster, or a cooperative grid.
 struct TeamLaunch {
     cudaLaunchConfig_t config = {};
     cudaLaunchAttribute attr[1] = {};
-    TeamLaunch(int grid, const ohm::KernelArgs &a, cudaStream_t stream) {
-        config.gridDim = dim3(grid);
-        config.blockDim = dim3(ohm::kSolverBlock);
+    TeamLaunch(const TeamShape &s, const ohm::KernelArgs &a, cudaStream_t stream) {
+        config.gridDim = dim3(s.grid);
+        config.blockDim = dim3(s.block);
         config.dynamicSmemBytes = (size_t)a.smem_bytes;
         config.stream = stream;
         if (a.cluster) {
             attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = grid;
+            attr[0].val.clusterDim.x = s.grid;
             attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
         } else {
             attr[0].id = cudaLaunchAttributeCooperative;

@@ -2,4 +2,4 @@
 #include "internal.cuh"
 
 template <>
-KernelFn persistent_kernel_for<1>() { return ohm::persistent_solver<1>; }
+KernelPair<KernelFn> persistent_kernel_for<1>() { return {ohm::persistent_solver<1>, ohm::persistent_solver_wide<1>}; }

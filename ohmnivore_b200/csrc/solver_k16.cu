@@ -2,4 +2,4 @@
 #include "internal.cuh"
 
 template <>
-KernelFn persistent_kernel_for<16>() { return ohm::persistent_solver<16>; }
+KernelPair<KernelFn> persistent_kernel_for<16>() { return {ohm::persistent_solver<16>, ohm::persistent_solver_wide<16>}; }

@@ -2,4 +2,4 @@
 #include "internal.cuh"
 
 template <>
-KernelFn persistent_kernel_for<32>() { return ohm::persistent_solver<32>; }
+KernelPair<KernelFn> persistent_kernel_for<32>() { return {ohm::persistent_solver<32>, ohm::persistent_solver_wide<32>}; }

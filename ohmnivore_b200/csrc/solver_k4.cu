@@ -2,4 +2,4 @@
 #include "internal.cuh"
 
 template <>
-KernelFn persistent_kernel_for<4>() { return ohm::persistent_solver<4>; }
+KernelPair<KernelFn> persistent_kernel_for<4>() { return {ohm::persistent_solver<4>, ohm::persistent_solver_wide<4>}; }

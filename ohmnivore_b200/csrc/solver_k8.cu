@@ -2,4 +2,4 @@
 #include "internal.cuh"
 
 template <>
-KernelFn persistent_kernel_for<8>() { return ohm::persistent_solver<8>; }
+KernelPair<KernelFn> persistent_kernel_for<8>() { return {ohm::persistent_solver<8>, ohm::persistent_solver_wide<8>}; }

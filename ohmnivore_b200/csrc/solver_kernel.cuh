@@ -65,6 +65,12 @@ enum PrecondKind : int { kPcAuto = 0, kPcJacobi = 1, kPcIsai = 2, kPcNone = 3 };
 #define OHM_SOLVER_BLOCK 512
 #endif
 constexpr int kSolverBlock = OHM_SOLVER_BLOCK;
+// Threads per block of its global-memory form (GlobalTeam): the phases of
+// krylov() and krylov_isai() wait for loads from L2 and HBM, and 512 threads
+// have too few in flight (us per iteration at 512 -> 1024 threads: 2000 x 2000
+// mesh 525 -> 357, the same in FP32 474 -> 288, 1000 x 1000 mesh in random order
+// 163 -> 113).
+constexpr int kWideBlock = 1024;
 
 // Breakdown test: |(a, b)| < kBreakdownRel * ||a|| ||b||.  The reference's
 // absolute 1e-30 (bicgstab.rs:107, :125) depends on the units of the
@@ -191,9 +197,11 @@ struct KernelArgs {
     // grid is one thread-block cluster.  slice_col and slice_val (5
     // entries per 4 nonzeros), slice_export (u8 per row), cself and rself (8
     // bytes per row) are that solve's workspace.
+    // scatter (host side): how far the rows of a block reach (ohm_scatter()).
     int smem_bytes;
     int64_t nnz_long;
     int cluster;
+    int scatter;
     uint16_t *slice_col;
     double *slice_val;
     uint8_t *slice_export;
@@ -227,7 +235,11 @@ struct SliceMap {
 // blocks is launched as one cluster and meets at cluster barriers with its
 // dot products exchanged through distributed shared memory; larger grids
 // meet at the counter barrier.  The sums have the same order in all three.
-struct GridTeam {
+// SLICES: whether the kernel has krylov_slice(); without it (kWideBlock
+// threads) the team works from global memory.
+template <bool SLICES>
+struct GridTeamT {
+    static constexpr bool kSlices = SLICES;
     int G, bid, r0, r1, gtid, gstride;
     double *smem;
     double *partials;
@@ -279,7 +291,13 @@ struct GridTeam {
     __device__ __forceinline__ bool allmax(double (&v)[NV]) { return reduce<NV, true>(v); }
 };
 
+using GridTeam = GridTeamT<true>;
+using GlobalTeam = GridTeamT<false>;
+template <class Team>
+constexpr int kTeamBlock = Team::kSlices ? kSolverBlock : kWideBlock;
+
 struct BlockTeam {
+    static constexpr bool kSlices = true;
     int r0, r1, gtid, gstride;
     double *smem;
     SliceMap map;
@@ -371,11 +389,11 @@ __device__ __forceinline__ void spmv_rows(const TR *__restrict__ rp, const TC *_
     }
 }
 
-// Block of the team that finishes team-shared work item q (GridTeam: block
+// Block of the team that finishes team-shared work item q (grid teams: block
 // q mod G; BlockTeam: its only block), and whether this block owns row i.
 template <class Team>
 __device__ __forceinline__ bool team_owns_item(const Team &g, int q) {
-    if constexpr (std::is_same<Team, GridTeam>::value) return q % g.G == g.bid;
+    if constexpr (!std::is_same<Team, BlockTeam>::value) return q % g.G == g.bid;
     else return true;
 }
 
@@ -874,7 +892,7 @@ __device__ __forceinline__ SliceOffsets slice_offsets(uint32_t R, uint32_t H, ui
 
 template <class Team>
 __device__ __forceinline__ bool team_of_one(const Team &g) {
-    if constexpr (std::is_same<Team, GridTeam>::value) return g.G == 1;
+    if constexpr (!std::is_same<Team, BlockTeam>::value) return g.G == 1;
     else return true;
 }
 
@@ -1528,16 +1546,18 @@ template <typename T, int LPR, class Team>
 __device__ __forceinline__ int krylov_any(const KernelArgs &a, Team &g, double tol_floor, double inner_rtol,
                                           int max_it, bool accept_partial, KrylovOut &out) {
     if (a.precond == kPcIsai) return krylov_isai<T, LPR>(a, g, tol_floor, inner_rtol, max_it, accept_partial, out);
-    if (g.map.state == kSliceNone && !slice_map<LPR>(a, g)) return kKrylovAbort;
-    if constexpr (LPR == 1) {
-        if (g.map.state == kSliceChip)
-            return krylov_slice<T, LPR, kSliceChip>(a, g, tol_floor, inner_rtol, max_it, accept_partial, out);
-        if (g.map.state == kSliceStream)
-            return krylov_slice<T, LPR, kSliceStream>(a, g, tol_floor, inner_rtol, max_it, accept_partial, out);
-    }
-    if constexpr (kHasCsr<LPR, Team>) {
-        if (g.map.state == kSliceCsr)
-            return krylov_slice<T, LPR, kSliceCsr>(a, g, tol_floor, inner_rtol, max_it, accept_partial, out);
+    if constexpr (Team::kSlices) {
+        if (g.map.state == kSliceNone && !slice_map<LPR>(a, g)) return kKrylovAbort;
+        if constexpr (LPR == 1) {
+            if (g.map.state == kSliceChip)
+                return krylov_slice<T, LPR, kSliceChip>(a, g, tol_floor, inner_rtol, max_it, accept_partial, out);
+            if (g.map.state == kSliceStream)
+                return krylov_slice<T, LPR, kSliceStream>(a, g, tol_floor, inner_rtol, max_it, accept_partial, out);
+        }
+        if constexpr (kHasCsr<LPR, Team>) {
+            if (g.map.state == kSliceCsr)
+                return krylov_slice<T, LPR, kSliceCsr>(a, g, tol_floor, inner_rtol, max_it, accept_partial, out);
+        }
     }
     return krylov<T, LPR>(a, g, tol_floor, inner_rtol, max_it, accept_partial, out);
 }
@@ -2025,6 +2045,12 @@ __device__ __forceinline__ bool solve_body(const KernelArgs &a, Team &g, DeviceI
 template <int LPR>
 __global__ void __launch_bounds__(kSolverBlock, 1) persistent_solver(const __grid_constant__ KernelArgs a) {
     GridTeam g;
+    g.init(a);
+    solve_body<LPR>(a, g, a.info);
+}
+template <int LPR>
+__global__ void __launch_bounds__(kWideBlock, 1) persistent_solver_wide(const __grid_constant__ KernelArgs a) {
+    GlobalTeam g;
     g.init(a);
     solve_body<LPR>(a, g, a.info);
 }

@@ -24,11 +24,11 @@ using namespace ohm;
 
 namespace {
 
-AdaptFn pick_adaptive(int lpr) {
+KernelPair<AdaptFn> pick_adaptive(int lpr) {
     return lpr == 1 ? adaptive_kernel_for<1>() : (lpr == 4 ? adaptive_kernel_for<4>() : adaptive_kernel_for<8>());
 }
 
-TranFn pick_tran(int lpr) {
+KernelPair<TranFn> pick_tran(int lpr) {
     return lpr == 1 ? transient_kernel_for<1>() : (lpr == 4 ? transient_kernel_for<4>() : transient_kernel_for<8>());
 }
 
@@ -235,9 +235,9 @@ static ohm_status tran_args(ohm_transient *t, double *x_dev, const ohm_newton_pa
 
 // Kernel arguments of a fixed-step run on x_dev with step h: the companion
 // base A = G + C/h is formed (and copied to the assembled arrays), the run
-// record zeroed.  Returns the kernel and grid to launch.
+// record zeroed.  Returns the kernel and its launch shape.
 static ohm_status tran_prepare(ohm_transient *t, double *x_dev, double h, const ohm_newton_params *np,
-                               KernelArgs &a, TranArgs &T, TranFn &fn, int &grid, const double *&G) {
+                               KernelArgs &a, TranArgs &T, TranFn &fn, TeamShape &shape, const double *&G) {
     ohm_ctx *c = t->ctx;
     ohm_status st = tran_args(t, x_dev, np, a, T, G);
     if (st != OHM_OK) return st;
@@ -249,17 +249,17 @@ static ohm_status tran_prepare(ohm_transient *t, double *x_dev, double h, const 
     }
     CUDA_TRY(cudaMemsetAsync(t->st, 0, sizeof(TranDev), c->stream));
     T.h = h;
-    fn = pick_tran(tran_lpr(t->n, nnz));
-    return ohm_team_shape((const void *)fn, c->num_sms, 0, true, nnz, a, grid);
+    return ohm_team_kernel(pick_tran(tran_lpr(t->n, nnz)), c->num_sms, 0, OHM_KRYLOV_LAYOUT_AUTO, nnz, a, shape, fn);
 }
 
 // One launch of steps [s0, s1).
-static cudaError_t tran_launch(ohm_ctx *c, TranFn fn, int grid, const KernelArgs &a, TranArgs T, int s0, int s1) {
+static cudaError_t tran_launch(ohm_ctx *c, TranFn fn, const TeamShape &shape, const KernelArgs &a, TranArgs T, int s0,
+                               int s1) {
     T.s0 = s0;
     T.s1 = s1;
     cudaError_t e = cudaMemsetAsync(c->sync_words, 0, 4 * sizeof(unsigned int), c->stream);
     if (e != cudaSuccess) return e;
-    TeamLaunch cfg(grid, a, c->stream);
+    TeamLaunch cfg(shape, a, c->stream);
     return cudaLaunchKernelEx(&cfg.config, fn, a, T);
 }
 
@@ -317,9 +317,9 @@ extern "C" ohm_status ohm_transient_run(ohm_transient *t, double *x_dev, double 
     KernelArgs a;
     TranArgs T;
     TranFn fn = nullptr;
-    int grid = 0;
+    TeamShape shape;
     const double *G = nullptr;
-    ohm_status st = tran_prepare(t, x_dev, h, np, a, T, fn, grid, G);
+    ohm_status st = tran_prepare(t, x_dev, h, np, a, T, fn, shape, G);
     if (st != OHM_OK) return st;
     T.t0 = t0;
     T.predict = t->predict;
@@ -330,7 +330,7 @@ extern "C" ohm_status ohm_transient_run(ohm_transient *t, double *x_dev, double 
     auto enqueue = [&]() -> cudaError_t {
         for (int l = 0; l < n_launch; ++l) {
             const int s0 = l * steps_per_launch;
-            cudaError_t e = tran_launch(c, fn, grid, a, T, s0, std::min(n_steps, s0 + steps_per_launch));
+            cudaError_t e = tran_launch(c, fn, shape, a, T, s0, std::min(n_steps, s0 + steps_per_launch));
             if (e != cudaSuccess) return e;
         }
         if (waveforms_host && need)
@@ -445,14 +445,15 @@ extern "C" ohm_status ohm_transient_run_adaptive(ohm_transient *t, double *x_dev
     P.fdev = t->ad_fdev;
     P.times = t->times;
     P.st = t->ad_st;
-    const AdaptFn fn = pick_adaptive(tran_lpr(t->n, t->nnz));
-    int grid = 0;
-    st = ohm_team_shape((const void *)fn, c->num_sms, 0, true, t->nnz, a, grid);
+    AdaptFn fn = nullptr;
+    TeamShape shape;
+    st = ohm_team_kernel(pick_adaptive(tran_lpr(t->n, t->nnz)), c->num_sms, 0, OHM_KRYLOV_LAYOUT_AUTO, t->nnz, a,
+                         shape, fn);
     if (st != OHM_OK) return st;
     CUDA_TRY(cudaMemsetAsync(t->ad_st, 0, sizeof(AdaptDev), c->stream));
     CUDA_TRY(cudaMemsetAsync(c->sync_words, 0, 4 * sizeof(unsigned int), c->stream));
     {
-        TeamLaunch cfg(grid, a, c->stream);
+        TeamLaunch cfg(shape, a, c->stream);
         CUDA_TRY(cudaLaunchKernelEx(&cfg.config, fn, a, T, P));
     }
     // restore the plan's assembled system to its conductance base
@@ -798,10 +799,10 @@ extern "C" ohm_status ohm_transient_adjoint(ohm_transient *t, const double *x0_d
     KernelArgs a;
     TranArgs T;
     TranFn fn = nullptr;
-    int grid = 0;
+    TeamShape shape;
     const double *G = nullptr;
     CUDA_TRY(cudaMemcpyAsync(x, x0_dev, n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
-    ohm_status st = tran_prepare(t, x, h, np, a, T, fn, grid, G);
+    ohm_status st = tran_prepare(t, x, h, np, a, T, fn, shape, G);
     if (st != OHM_OK) return st;
     T.t0 = t0;
     T.n_probes = 0;
@@ -812,7 +813,7 @@ extern "C" ohm_status ohm_transient_adjoint(ohm_transient *t, const double *x0_d
     }
     for (int sg = 0; sg < nseg; ++sg) {
         CUDA_TRY(cudaMemcpyAsync(ck + (size_t)sg * n, x, n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
-        CUDA_TRY(tran_launch(c, fn, grid, a, T, sg * K, std::min(n_steps, (sg + 1) * K)));
+        CUDA_TRY(tran_launch(c, fn, shape, a, T, sg * K, std::min(n_steps, (sg + 1) * K)));
     }
     TranDev d{};
     st = tran_status(t, t0, h, d);
@@ -831,7 +832,7 @@ extern "C" ohm_status ohm_transient_adjoint(ohm_transient *t, const double *x0_d
                                      c->stream));
             T.states = S;
             T.state_base = s0;
-            CUDA_TRY(tran_launch(c, fn, grid, a, T, s0, s1));
+            CUDA_TRY(tran_launch(c, fn, shape, a, T, s0, s1));
             ++launches;
             st = tran_status(t, t0, h, d);
         }

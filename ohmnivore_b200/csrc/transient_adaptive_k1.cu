@@ -4,6 +4,8 @@
 namespace ohm {
 
 template <>
-AdaptFn adaptive_kernel_for<1>() { return adaptive_kernel<1>; }
+KernelPair<AdaptFn> adaptive_kernel_for<1>() {
+    return {adaptive_kernel<1, GridTeam>, adaptive_kernel<1, GlobalTeam>};
+}
 
 }  // namespace ohm

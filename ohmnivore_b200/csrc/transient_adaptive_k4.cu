@@ -4,6 +4,8 @@
 namespace ohm {
 
 template <>
-AdaptFn adaptive_kernel_for<4>() { return adaptive_kernel<4>; }
+KernelPair<AdaptFn> adaptive_kernel_for<4>() {
+    return {adaptive_kernel<4, GridTeam>, adaptive_kernel<4, GlobalTeam>};
+}
 
 }  // namespace ohm

@@ -4,6 +4,8 @@
 namespace ohm {
 
 template <>
-AdaptFn adaptive_kernel_for<8>() { return adaptive_kernel<8>; }
+KernelPair<AdaptFn> adaptive_kernel_for<8>() {
+    return {adaptive_kernel<8, GridTeam>, adaptive_kernel<8, GlobalTeam>};
+}
 
 }  // namespace ohm

@@ -4,6 +4,8 @@
 namespace ohm {
 
 template <>
-TranFn transient_kernel_for<1>() { return transient_kernel<1>; }
+KernelPair<TranFn> transient_kernel_for<1>() {
+    return {transient_kernel<1, GridTeam>, transient_kernel<1, GlobalTeam>};
+}
 
 }  // namespace ohm

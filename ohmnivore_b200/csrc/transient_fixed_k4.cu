@@ -4,6 +4,8 @@
 namespace ohm {
 
 template <>
-TranFn transient_kernel_for<4>() { return transient_kernel<4>; }
+KernelPair<TranFn> transient_kernel_for<4>() {
+    return {transient_kernel<4, GridTeam>, transient_kernel<4, GlobalTeam>};
+}
 
 }  // namespace ohm

@@ -4,6 +4,8 @@
 namespace ohm {
 
 template <>
-TranFn transient_kernel_for<8>() { return transient_kernel<8>; }
+KernelPair<TranFn> transient_kernel_for<8>() {
+    return {transient_kernel<8, GridTeam>, transient_kernel<8, GlobalTeam>};
+}
 
 }  // namespace ohm

@@ -86,10 +86,10 @@ __device__ __forceinline__ double source_value(const ohm_source &s, double t, co
     }
 }
 
-template <int LPR>
-__global__ void __launch_bounds__(kSolverBlock, 1) transient_kernel(const __grid_constant__ KernelArgs a,
+template <int LPR, class Team>
+__global__ void __launch_bounds__(kTeamBlock<Team>, 1) transient_kernel(const __grid_constant__ KernelArgs a,
                                                                      const __grid_constant__ TranArgs T) {
-    GridTeam g;
+    Team g;
     g.init(a);
     if (T.st->status != 0) return;     // an earlier chunk failed (uniform: written before this launch)
     const double inv_h = 1.0 / T.h;
@@ -183,11 +183,11 @@ struct AdaptArgs {
     AdaptDev *st;
 };
 
-template <int LPR>
-__global__ void __launch_bounds__(kSolverBlock, 1) adaptive_kernel(const __grid_constant__ KernelArgs a,
+template <int LPR, class Team>
+__global__ void __launch_bounds__(kTeamBlock<Team>, 1) adaptive_kernel(const __grid_constant__ KernelArgs a,
                                                                     const __grid_constant__ TranArgs T,
                                                                     const __grid_constant__ AdaptArgs P) {
-    GridTeam g;
+    Team g;
     g.init(a);
     const int r0 = g.r0, r1 = g.r1;
     const double h_min = P.tstep / 10000.0, h_max = P.tstep, lte_tol = 1e-3;
@@ -343,22 +343,22 @@ __global__ void __launch_bounds__(kSolverBlock, 1) adaptive_kernel(const __grid_
 using TranFn = void (*)(KernelArgs, TranArgs);
 using AdaptFn = void (*)(KernelArgs, TranArgs, AdaptArgs);
 
-// Kernels for lanes per row 1, 4 or 8.
+// Kernels for lanes per row 1, 4 or 8, with and without Krylov slices.
 template <int LPR>
-TranFn transient_kernel_for();
+KernelPair<TranFn> transient_kernel_for();
 template <int LPR>
-AdaptFn adaptive_kernel_for();
+KernelPair<AdaptFn> adaptive_kernel_for();
 template <>
-TranFn transient_kernel_for<1>();
+KernelPair<TranFn> transient_kernel_for<1>();
 template <>
-TranFn transient_kernel_for<4>();
+KernelPair<TranFn> transient_kernel_for<4>();
 template <>
-TranFn transient_kernel_for<8>();
+KernelPair<TranFn> transient_kernel_for<8>();
 template <>
-AdaptFn adaptive_kernel_for<1>();
+KernelPair<AdaptFn> adaptive_kernel_for<1>();
 template <>
-AdaptFn adaptive_kernel_for<4>();
+KernelPair<AdaptFn> adaptive_kernel_for<4>();
 template <>
-AdaptFn adaptive_kernel_for<8>();
+KernelPair<AdaptFn> adaptive_kernel_for<8>();
 
 }  // namespace ohm
