@@ -33,6 +33,7 @@ struct ohm_batch {
     // instances solved one at a time by the whole GPU (ohm_batch_set_split).
     std::vector<InstanceOffsets> h_offsets;
     std::vector<int8_t> scatter;        // per instance (ohm_scatter())
+    std::vector<uint32_t> widths;       // per instance: sum of its 32-row slices' longest rows
     std::vector<int32_t> h_order;
     double *team_partials = nullptr;   // reduction partials of those solves
     int split = 1;
@@ -80,6 +81,7 @@ extern "C" ohm_status ohm_batch_create(ohm_ctx *c, int64_t n_inst, const int64_t
     std::vector<uint32_t> diag(rows), off(rows);
     std::vector<uint8_t> flag(rows), sflag(rows);
     std::vector<int8_t> scatter(n_inst, kScatterNear);
+    std::vector<uint32_t> widths(n_inst, 0);
     bool any_pair = false;
     int64_t max_nnz_row = 0;
     for (int64_t i = 0; i < n_inst; ++i) {
@@ -139,6 +141,11 @@ extern "C" ohm_status ohm_batch_create(ohm_ctx *c, int64_t n_inst, const int64_t
         any_pair |= pc.any_pair;
         scatter[i] = (int8_t)ohm_scatter(n, dn + qn + mn, c->num_sms, rp, cl);
         for (int64_t r = 0; r < n; ++r) max_nnz_row = std::max<int64_t>(max_nnz_row, rp[r + 1] - rp[r]);
+        for (int64_t r = 0; r < n; r += 32) {
+            uint32_t w = 0;
+            for (int64_t k = r; k < std::min(n, r + 32); ++k) w = std::max(w, rp[k + 1] - rp[k]);
+            widths[i] += w;
+        }
     }
     // longest first
     std::vector<int32_t> order(n_inst);
@@ -228,6 +235,7 @@ extern "C" ohm_status ohm_batch_create(ohm_ctx *c, int64_t n_inst, const int64_t
     b->host_infos.resize(n_inst);
     b->h_order = order;
     b->scatter = scatter;
+    b->widths = widths;
     b->h_offsets.resize(n_inst);
     for (int64_t i = 0; i < n_inst; ++i) {
         InstanceOffsets &o = b->h_offsets[i];
@@ -291,8 +299,11 @@ static ohm_status batch_args(ohm_batch *b, double *x_dev, const ohm_newton_param
 
 // Dynamic shared memory of a block: an equal share of an SM's, less where the
 // largest circuit needs less.  A circuit whose slice does not fit keeps its
-// gather vector and as many of its vectors there as do (krylov_slice()).
-static int batch_smem_bytes(ohm_batch *b, BatchFn fn, int shape) {
+// gather vector and as many of its vectors there as do (krylov_slice()).  None
+// where most of the work (rows^1.5, see split_instances()) is in circuits that
+// cannot use it, their rows too uneven to pad: krylov() wants it as L1 (300
+// circuits of 1,000 rows, one of them 300 entries long: 73 -> 41 ms).
+static int batch_smem_bytes(const ohm_batch *b, BatchFn fn, int lpr, int shape) {
     int dev = 0, sm_total = 0;
     cudaFuncAttributes fa{};
     if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -307,7 +318,18 @@ static int batch_smem_bytes(ohm_batch *b, BatchFn fn, int shape) {
         const int64_t n = o.ro1 - o.ro, z = o.no1 - o.no;
         need = std::max(need, n * (9 * 8 + 1) + n / 8 + (z + z / 4) * (8 + 2) + 512);
     }
-    return (int)std::max<int64_t>(0, std::min(share, need) & ~(int64_t)15);
+    const int64_t bytes = std::max<int64_t>(0, std::min(share, need) & ~(int64_t)15);
+    double total = 0.0, slices = 0.0;
+    for (size_t i = 0; i < b->h_offsets.size(); ++i) {
+        const InstanceOffsets &o = b->h_offsets[i];
+        const int64_t n = o.ro1 - o.ro, z = o.no1 - o.no, w = b->widths[i];
+        const double work = (double)n * std::sqrt((double)n);
+        total += work;
+        const bool even = lpr > 1 || 32 * w <= z + z / 4 ||
+                          (w <= 0xFFFF && slice_offsets((uint32_t)n, 0, (uint32_t)w, false).end <= bytes);
+        if (n < 0xFFFF && even && slice_offsets((uint32_t)n, 0, 0, lpr > 1).vec <= bytes) slices += work;
+    }
+    return 2.0 * slices >= total ? (int)bytes : 0;
 }
 
 // One launch over `n` instances listed in `order` (device): a persistent grid
@@ -318,7 +340,7 @@ static ohm_status launch_batch(ohm_batch *b, BatchArgs B, int lpr, int shape, in
     B.n_inst = n;
     BatchFn fn = batch_kernel(lpr, shape);
     const int block = kBatchShapes[shape].block;
-    B.base.smem_bytes = batch_smem_bytes(b, fn, shape);
+    B.base.smem_bytes = batch_smem_bytes(b, fn, lpr, shape);
     int per_sm = 0;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, block, B.base.smem_bytes));
     if (per_sm < 1) return ohm_fail(OHM_ERR_CUDA, "batch kernel does not fit on an SM");

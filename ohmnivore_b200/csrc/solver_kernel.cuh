@@ -868,7 +868,7 @@ namespace ohm {
 constexpr uint32_t kHaloPaired = 0x80000000u;    // halo entry: the row is half of a 2x2 pair
 constexpr uint8_t kRowPaired = 1, kRowExport = 2, kRowLong = 4;
 
-__device__ __forceinline__ uint32_t up16(uint32_t x) { return (x + 15u) & ~15u; }
+__host__ __device__ __forceinline__ uint32_t up16(uint32_t x) { return (x + 15u) & ~15u; }
 
 // Byte offsets in dynamic shared memory: slice starts at 0 (csr: the rows'
 // first nonzeros), halo list, row flags, columns of the matrix slices (32 W entries; none when they are in
@@ -877,7 +877,7 @@ __device__ __forceinline__ uint32_t up16(uint32_t x) { return (x + 15u) & ~15u; 
 struct SliceOffsets {
     uint32_t halo, flag, col, z, vec, vec_bytes, val, end;
 };
-__device__ __forceinline__ SliceOffsets slice_offsets(uint32_t R, uint32_t H, uint32_t W, bool csr) {
+__host__ __device__ __forceinline__ SliceOffsets slice_offsets(uint32_t R, uint32_t H, uint32_t W, bool csr) {
     SliceOffsets o;
     o.halo = up16(4u * ((csr ? R : (R + 31u) / 32u) + 1u));
     o.flag = o.halo + up16(4u * H);
