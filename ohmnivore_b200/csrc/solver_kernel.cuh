@@ -1426,8 +1426,21 @@ __device__ __forceinline__ int krylov_slice(const KernelArgs &a, Team &g, double
                         y += (Acc)lval[k + 64u] * (Acc)z2;
                         y += (Acc)lval[k + 96u] * (Acc)z3;
                     }
+                    if (MODE == kSliceStream && sl[s + 1] - sl[s] < 4u) {
+                        // short rows (a ladder's) from global memory in one
+                        // round trip, not one per entry
+                        if (k < e) {
+                            const bool b1 = k + 32u < e, b2 = k + 64u < e;
+                            const uint16_t c0 = lcol[k], c1 = b1 ? lcol[k + 32u] : c0, c2 = b2 ? lcol[k + 64u] : c0;
+                            const T v0 = lval[k], v1 = b1 ? lval[k + 32u] : T(0), v2 = b2 ? lval[k + 64u] : T(0);
+                            y += (Acc)v0 * (Acc)z[c0];
+                            if (b1) y += (Acc)v1 * (Acc)z[c1];
+                            if (b2) y += (Acc)v2 * (Acc)z[c2];
+                        }
+                    } else {
 #pragma unroll 1
-                    for (; k < e; k += 32u) y += (Acc)lval[k] * (Acc)z[lcol[k]];
+                        for (; k < e; k += 32u) y += (Acc)lval[k] * (Acc)z[lcol[k]];
+                    }
                     if (li < R && !(has_long && (flag[li] & kRowLong))) row(r0 + li, (double)y);
                 }
             }
