@@ -496,8 +496,16 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *s
 // shadow residual).  Such breakdowns come after a spike of the recurrence; 4
 // of 440 solves of a 600 x 600 diode mesh (1.0 V, 5 % diodes) met one, at 140 to
 // 2.6e8 times the initial residual, and one of them then spent the rest of its
-// 20,000 iterations above it.
+// 20,000 iterations above it.  FP64 solves only (the FP32 attempts have few
+// iterations and an FP64 solve after them), and only where no DC continuation
+// follows a failure: its direct attempts often cannot succeed, and trying them
+// longer took most of a batch's time (ten batches of 512 amplifiers 1.40 -> 1.89
+// s).
 constexpr double kRestartFromStart = 100.0;
+template <typename T>
+__device__ __forceinline__ bool restarts_from_start(const KernelArgs &a) {
+    return sizeof(T) == 8 && a.continuation == 0;
+}
 
 // |x| < rel sqrt(y), compared as squares: a square root is 120 cycles on the
 // one lane that every thread waits for.  Where a square would leave the
@@ -652,11 +660,12 @@ __device__ __forceinline__ int krylov(const KernelArgs &a, Team &g, double tol_f
             if (!isfinite(r0norm)) { code = kKrylovNan; break; }
             if (r0norm < abs_tol || r0norm == 0.0) { code = kKrylovConverged; break; }
         }
+        const bool try_start = restarts_from_start<T>(a);
         bool back = false;
         for (; it < max_it; ++it) {
             if (below_root(rho_new, kBreakdownRel, rhat2 * rr_cur)) {
                 if (out.restarts < a.max_restarts && rr_cur > 0.0) {
-                    back = !again && rw_cur > kRestartFromStart * rw0;
+                    back = try_start && !again && rw_cur > kRestartFromStart * rw0;
                     if (back) break;
                     OHM_RESTART();
                 } else {
@@ -707,7 +716,7 @@ __device__ __forceinline__ int krylov(const KernelArgs &a, Team &g, double tol_f
                         code = kKrylovMaxIter;
                         break;
                     }
-                    back = !again && rw_cur > kRestartFromStart * rw0;
+                    back = try_start && !again && rw_cur > kRestartFromStart * rw0;
                     if (back) { ++it; break; }
                     OHM_RESTART();        // cur still holds r; restart from it
                     continue;
@@ -1080,7 +1089,7 @@ struct KrylovScalars {
 struct KrylovLimits {
     double tol_floor, inner_rtol;
     int max_it, max_restarts;
-    bool accept_partial;
+    bool accept_partial, try_start;
 };
 __device__ __forceinline__ void krylov_scalars_step(KrylovScalars &q, const double (&s)[4], const KrylovLimits &lim) {
     bool top = false, restart = false, back = false;
@@ -1157,7 +1166,7 @@ __device__ __forceinline__ void krylov_scalars_step(KrylovScalars &q, const doub
             else code = kKrylovBreakRho;
         }
         if (stop) code = kKrylovMaxIter;
-        back = restart && !stop && !q.again && q.rw > kRestartFromStart * q.rw0;
+        back = restart && !stop && lim.try_start && !q.again && q.rw > kRestartFromStart * q.rw0;
         if (back) {
             ++q.restarts;
             q.again = 1;
@@ -1270,7 +1279,7 @@ __device__ __forceinline__ int krylov_slice(const KernelArgs &a, Team &g, double
         if constexpr (MODE == kSliceChip) return (const uint16_t *)(ohm_dsmem + o.col);
         else return V.lcol;
     };
-    const KrylovLimits lim{tol_floor, inner_rtol, max_it, a.max_restarts, accept_partial};
+    const KrylovLimits lim{tol_floor, inner_rtol, max_it, a.max_restarts, accept_partial, restarts_from_start<T>(a)};
 
     for (;;) {
         const int phase = S.phase;
