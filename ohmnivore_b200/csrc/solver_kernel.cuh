@@ -566,7 +566,9 @@ __device__ __forceinline__ int krylov(const KernelArgs &a, Team &g, double tol_f
     T *s_pair = (T *)a.s;   // s of the rows of 2x2 pairs (read by the partner in E)
     double *w = a.dx + r0;
     auto own = [&](KRec<T> *buf, int i) -> KRec<T> { return buf[i]; };
-    auto is_paired = [&](int i) -> bool { return partner[i] >= 0; };
+    // (as in krylov_slice(): with other preconditioners its blocks leave no s_pair)
+    const bool pairs = a.precond == kPcAuto;
+    auto is_paired = [&](int i) -> bool { return pairs && partner[i] >= 0; };
 
     double r0norm = 0.0, abs_tol = 0.0, tol2 = 0.0;     // stopping norm (scaled for Newton)
     double rr0 = 0.0, rw0 = 0.0;
