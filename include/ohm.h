@@ -286,8 +286,9 @@ ohm_status ohm_plan_limit(ohm_plan *plan, const double *x_old_host, double *x_ne
  * AC sweep (src/analysis/ac.rs:25-78): for every frequency f solve
  * (G + j 2 pi f C) x = b_ac (sparse.rs:149-178 forms the matrix; gpu.rs:210-700
  * is the reference's complex Jacobi BiCGSTAB, one frequency at a time).  Here
- * all points are solved by one launch, one thread block per point, in FP64
- * complex arithmetic.  c_values lie on the pattern of g_values (NULL: no C);
+ * all points are solved by one launch, in FP64 complex arithmetic: a
+ * thread-block cluster per point where its shared memory holds the point's
+ * part, else one thread block, or a team of blocks, per point.  c_values lie on the pattern of g_values (NULL: no C);
  * b and x are interleaved (re, im); x_re_im holds n_freq x n complex values.
  * Like the reference, the devices are not linearised: pass the Jacobian
  * values of a DC operating point as g_values for a small-signal analysis.
@@ -406,7 +407,7 @@ ohm_status ohm_transient_set_predictor(ohm_transient *tr, int32_t order);
  * times_host (max_points doubles) and waveforms_host (max_points x n_probes,
  * row-major), either may be NULL; info->points counts them all, so a run
  * with info->points > max_points was truncated and can be repeated with a
- * larger capacity.  The whole run is one cooperative launch.  Errors:
+ * larger capacity.  The whole run is one launch.  Errors:
  * OHM_ERR_TIMESTEP as transient.rs:128-133, a failed Newton solve as in
  * ohm_transient_run (info->failed_solve 1 = TRAP, 2 = BE). */
 typedef struct {

@@ -17,6 +17,10 @@ constexpr int kStatusTimeout = 5;
 // kTightSpins, then __nanosleep(64)); about 2-3 s in total.  A wait that runs
 // out records kStatusTimeout and the kernel returns; with a cooperative launch
 // every block is resident, so a healthy barrier never comes near the bound.
+// Clusters wait at the hardware's barrier, which has no bound to set: their
+// blocks are scheduled together, take the same branches (decided on reductions
+// that are bit-identical in every block) and leave only at the same points, and
+// the barrier does not count threads that have left.
 constexpr uint32_t kBarrierSpinLimit = 1u << 22;
 constexpr uint32_t kTightSpins = 2048;
 
@@ -133,8 +137,8 @@ template <int NV>
 __device__ __forceinline__ void block_max(double (&v)[NV], double *smem) { block_allreduce<NV, true>(v, smem); }
 
 // Cluster barrier (release / acquire, every thread of every block of the
-// cluster): 0.33 us for 2 to 16 blocks of 1024 threads, against 1.0-1.13 us
-// for the counter barrier above.
+// cluster): 0.33 us for 2 to 16 blocks, against 1.0-1.13 us for the counter
+// barrier below.
 __device__ __forceinline__ void cluster_barrier() {
     __syncwarp();       // the aligned forms want the whole warp together
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");

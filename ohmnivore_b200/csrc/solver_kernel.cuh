@@ -1,7 +1,8 @@
 // Persistent solver kernel: the whole Newton loop (device evaluation, MNA
 // stamping through the stamp map, FP64 residual, right-preconditioned
 // BiCGSTAB, voltage limiting, convergence test) or a linear solve with FP64
-// iterative refinement, in ONE cooperative launch.
+// iterative refinement, in ONE launch: a block, a thread-block cluster or a
+// cooperative grid.
 //
 // Algorithms followed:
 //   Newton loop       src/solver/newton.rs:153-488 (newton_solve)
@@ -21,9 +22,9 @@
 // Work split: block b owns rows [b*n/G, (b+1)*n/G).  Vector phases map one
 // thread per row; SpMV phases map LPR lanes per row (sub-warp CSR).  Device
 // phases are grid-strided over devices / touched slots.  Phases are separated
-// by a bounded grid barrier; dot products are reduced deterministically
-// (per-block partials, then every block sums all partials in one fixed order),
-// so all blocks hold bit-identical scalars and take the same branch.
+// by team synchronisations (GridTeam); dot products are reduced
+// deterministically (per-block values, then every block sums them all in one
+// fixed order), so all blocks hold bit-identical scalars and take the same branch.
 #pragma once
 
 #include <cstdint>
@@ -61,10 +62,7 @@ enum PrecondKind : int { kPcAuto = 0, kPcJacobi = 1, kPcIsai = 2, kPcNone = 3 };
 // reductions, address arithmetic) of 1024 threads with 64: DC of the 500 x 500
 // diode mesh 382 -> 234 ms, of a 100 x 100 one 31.7 -> 24.7 ms (256 threads:
 // 276 and 26.5 ms).
-#ifndef OHM_SOLVER_BLOCK
-#define OHM_SOLVER_BLOCK 512
-#endif
-constexpr int kSolverBlock = OHM_SOLVER_BLOCK;
+constexpr int kSolverBlock = 512;
 // Threads per block of its global-memory form (GlobalTeam): the phases of
 // krylov() and krylov_isai() wait for loads from L2 and HBM, and 512 threads
 // have too few in flight (us per iteration at 512 -> 1024 threads: 2000 x 2000
