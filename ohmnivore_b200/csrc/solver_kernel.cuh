@@ -863,7 +863,7 @@ namespace ohm {
 //   stream (larger slices) z and the vectors, in the order of their traffic,
 //          while they fit; the 32-row slices of the matrix in global memory,
 //          the values of as many as still fit on the chip (600 x 600 mesh,
-//          2,432 rows a block: 547 -> 537 ms);
+//          2,432 rows a block: 2 % of a solve);
 //   csr    (several lanes per row, or rows too uneven to pad) vectors as in
 //          `stream`; the matrix in compact rows with local column indices, on
 //          the chip where it fits.  Blocks with a few long rows: without it they

@@ -1,6 +1,7 @@
 // Fixed-step backward-Euler transient with a Newton solve per step.
 //
-// One persistent cooperative kernel runs a chunk of steps; per step the grid
+// One persistent kernel (a block, a cluster or a cooperative grid) runs a chunk of
+// steps; per step the team
 //   1. forms the BE right-hand side b_n = b(t_n) + (C/h) x_{n-1}
 //      (transient.rs:326-333) with the sources evaluated on the device
 //      (transient_source.rs:8-118), C in its own compact CSR,
